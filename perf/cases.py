@@ -212,3 +212,147 @@ def tolerance(case):
     layers 5e-3 to 8e-3 and 0.05, gradients (the first moment) 6e-3 to 1e-2 and 0.34, second moments 1.1e-2."""
     return {"train": {"rel": 3e-2, "max": 0.99}, "logits": {"rel": 3e-2, "max": 0.2},
             "linear": {"rel": 7e-3, "max": 2e-2}}.get(case["kind"], {"rel": 1e-2, "max": 0.4})
+
+
+# ------------------------------------------------------------------------------------------------
+# The same passes in 64 bits, in plain torch
+# ------------------------------------------------------------------------------------------------
+
+
+def _visible(case, row0, row1, device):
+    """Indices of the keys that rows [row0, row1) may see, and which of them each row sees (None: all of them)."""
+    S = case["seq"]
+    if case["kind"] in ("train", "logits", "attention", "fp8kv"):
+        if not case.get("causal", True):
+            return torch.arange(S, device=device), None
+        keys, window, every = torch.arange(row1, device=device), 0, 0
+    else:
+        window, every = case["window"] // 128, case["global_every"]
+        keys = torch.arange(row1, device=device)
+        keep = keys // 128 > row0 // 128 - window
+        keys = keys[keep | (keys // 128 % every == 0)] if every else keys[keep]
+    rows = torch.arange(row0, row1, device=device)[:, None]
+    mask = keys[None] <= rows
+    if window:
+        near = rows // 128 - keys[None] // 128 < window
+        mask &= (near | (keys[None] // 128 % every == 0)) if every else near
+    return keys, mask
+
+
+class _Attend64(torch.autograd.Function):
+    """softmax(Q K^T / sqrt(d)) V, some rows of one KV head's query heads at a time."""
+
+    @staticmethod
+    def _pieces(case, q, k):
+        B, S, Hq, _ = q.shape
+        step = max(128, min(1024, 2 ** 28 // (S * (Hq // k.shape[2])) // 128 * 128))
+        for r0 in range(0, S, step):
+            r1 = min(S, r0 + step)
+            keys, mask = _visible(case, r0, r1, q.device)
+            for b in range(B):
+                for h in range(k.shape[2]):
+                    G = Hq // k.shape[2]
+                    yield b, slice(r0, r1), slice(h * G, (h + 1) * G), h, keys, mask
+
+    @staticmethod
+    def _p(q, k, piece):
+        b, rows, heads, h, keys, mask = piece
+        s = q[b, rows, heads].transpose(0, 1) @ k[b, keys, h].T * HEAD_DIM ** -0.5     # [G, rows, keys]
+        return torch.softmax(s if mask is None else s.masked_fill_(~mask, -math.inf), -1)
+
+    @staticmethod
+    def forward(ctx, q, k, v, case):
+        o = torch.empty_like(q)
+        for piece in _Attend64._pieces(case, q, k):
+            b, rows, heads, h, keys, _ = piece
+            o[b, rows, heads] = (_Attend64._p(q, k, piece) @ v[b, keys, h]).transpose(0, 1)
+        ctx.save_for_backward(q, k, v)
+        ctx.case = case
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v = ctx.saved_tensors
+        dq, dk, dv = torch.empty_like(q), torch.zeros_like(k), torch.zeros_like(v)
+        for piece in _Attend64._pieces(ctx.case, q, k):
+            b, rows, heads, h, keys, _ = piece
+            p, g = _Attend64._p(q, k, piece), do[b, rows, heads].transpose(0, 1)
+            dv[b, :, h].index_add_(0, keys, torch.einsum("grk,grd->kd", p, g))
+            dp = g @ v[b, keys, h].T
+            ds = p.mul_(dp - (dp * p).sum(-1, keepdim=True)).mul_(HEAD_DIM ** -0.5)
+            dq[b, rows, heads] = (ds @ k[b, keys, h]).transpose(0, 1)
+            dk[b, :, h].index_add_(0, keys, torch.einsum("grk,grd->kd", ds, q[b, rows, heads].transpose(0, 1)))
+        return dq, dk, dv, None
+
+
+def _hidden64(case, w, tokens):
+    """The hidden states in front of the LM head; w: name -> weight in 64 bits."""
+    cfg = _config(case)
+    B, S = tokens.shape
+    inv = cfg.rope_theta ** (-torch.arange(0, HEAD_DIM, 2, device="cuda", dtype=torch.float64) / HEAD_DIM)
+    angle = torch.arange(S, device="cuda", dtype=torch.float64)[:, None] * inv
+    cos, sin = angle.cos()[:, None], angle.sin()[:, None]
+
+    def norm(x, weight):
+        return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + cfg.norm_eps) * weight
+
+    def rotate(x):
+        a, b = x.chunk(2, -1)
+        return torch.cat([a * cos - b * sin, b * cos + a * sin], -1)
+
+    h = w["embed.weight"][tokens]
+    for n in range(cfg.n_layers):
+        p = "layers.%d." % n
+        qkv = (norm(h, w[p + "norm1"]) @ w[p + "wqkv"].T).view(B, S, -1, HEAD_DIM)
+        q, k, v = qkv.split([cfg.n_heads, cfg.n_kv_heads, cfg.n_kv_heads], 2)
+        h = h + _Attend64.apply(rotate(q), rotate(k), v, case).reshape(B, S, -1) @ w[p + "wo"].T
+        gate, up = (norm(h, w[p + "norm2"]) @ w[p + "wgu"].T).chunk(2, -1)
+        h = h + (torch.nn.functional.silu(gate) * up) @ w[p + "wd"].T
+    return norm(h, w["final_norm"])
+
+
+def _exact_train(case, state):
+    flat = state["trainer"].model.flat
+    index, decay_end, total = dict(flat.index), flat.decay_end, flat.total
+    params = flat.params.double()
+    tokens, targets = state["tokens"].cuda(), state["targets"].cuda()
+    state.clear()
+    w = {n: params[o: o + math.prod(s)].view(s).requires_grad_(True) for n, (o, s) in index.items()}
+    loss = torch.nn.functional.cross_entropy((_hidden64(case, w, tokens) @ w["lm_head.weight"].T).flatten(0, 1),
+                                             targets.flatten())
+    grads = torch.autograd.grad(loss, list(w.values()))
+    g = torch.zeros(total, device="cuda", dtype=torch.float64)
+    for (o, s), x in zip(index.values(), grads):
+        g[o: o + math.prod(s)] = x.flatten()
+    g *= min(1.0, 1.0 / (float(g.norm()) + 1e-6))
+    params = params.detach()
+    params[:decay_end] *= 1 - 3e-4 * 0.1
+    return dict(loss=float(loss), params=params - 3e-4 * g / (g.abs() + 1e-8), m=0.1 * g, v=0.05 * g * g)
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "train" and work(case)["flops"] > 1.2e14:   # too long in 64 bits
+        return None
+    state = prepare(case, seed)
+    if kind == "train":
+        return _exact_train(case, state)
+    if kind == "logits":
+        flat = state["model"].flat
+        w = {n: flat.param(n).double() for n in flat.index}
+        with torch.no_grad():
+            return _hidden64(case, w, state["tokens"]) @ w["lm_head.weight"].T
+    wide = {n: x.detach().double() for n, x in state.items() if isinstance(x, torch.Tensor)}
+    if kind == "linear":
+        x, w, dy = wide["x"], wide["w"], wide["grad"]
+        return x @ w.T + wide["residual"], dy @ w, dy.T @ x, dy
+    if kind == "fp8kv":   # e4m3 codes with one 32-bit scale per head and 128 tokens are the format, not its error
+        for n in "kv":
+            x = state[n].float().unflatten(1, (-1, 128))
+            scale = x.abs().amax((2, 4), keepdim=True) / 448
+            wide[n] = ((x * (1 / scale)).to(torch.float8_e4m3fn).double() * scale.double()).flatten(1, 2)
+    qkv = [wide[n].requires_grad_(True) for n in "qkv"]
+    o = _Attend64.apply(*qkv, case)
+    if kind == "fp8kv" or state["grad"] is None:
+        return o.detach()
+    return (o.detach(), *torch.autograd.grad(o, qkv, wide["grad"]))
