@@ -18,6 +18,7 @@
 #include "../common/tma_host.h"
 #include "attn.h"
 #include "tile_iter.cuh"
+#include "work_order.h"
 
 namespace zx {
 
@@ -29,6 +30,7 @@ constexpr int HD = 128;
 constexpr int BT = 128;                    // tile edge in tokens (both Q and KV)
 constexpr int TILE_BYTES = BT * HD * 2;    // 32 KB
 constexpr int HALF_BYTES = TILE_BYTES / 2; // one 64-wide d chunk
+constexpr int HALF_Q = 64 * 128;           // 64 rows of a d chunk: start of a tile's second half of tokens
 constexpr int NUM_THREADS = 352;           // dQ kernel: 8 compute warps (two warpgroups) + TMA warp + two MMA warps
 constexpr int W_TMA = 8, W_MMA = 9, W_MMA_DQ = 10;   // dQ kernel roles (the dK/dV kernel has its own, below)
 constexpr int N_COMPUTE = 256;             // compute threads
@@ -54,6 +56,7 @@ struct BwdParams {
   int causal, window_blocks, global_every;
   int n_q_tiles, n_kv_tiles;
   int q_tiles_per_chunk, kv_tiles_per_chunk;
+  int kv_heads_per_group, q_heads_per_group;   // block order, see work_item
   int q_chunk_pos[kAttnMaxChunks];
   int kv_chunk_pos[kAttnMaxChunks];
   const float* lse;
@@ -84,7 +87,6 @@ struct BwdParams {
 #define ZX_TRACE_DKDV(iter, slot) do { } while (0)
 #define ZX_TRACE(iter, slot) do { } while (0)
 #endif
-#define ZX_TRACE_W(iter, k) do { } while (0)
 
 __device__ __forceinline__ int q_tile_pos(const BwdParams& p, int t) {
   return p.q_chunk_pos[t / p.q_tiles_per_chunk] + (t % p.q_tiles_per_chunk) * BT;
@@ -188,13 +190,14 @@ constexpr int Q_STAGES = 3, DO_STAGES = 2;
 // exponential phase is bound by the special-function unit whatever the warp count; everything
 // around it (TMEM round trips, barrier latency, the dS arithmetic) is per-warp serial time, and
 // four warps per scheduler overlap it where two could not.
-constexpr int KW_COMPUTE = 16, KW_TMA = 16, KW_MMA = 17, KW_PULL = 18;
-constexpr int DKDV_THREADS = (KW_COMPUTE + 3) * 32;
+constexpr int KW_COMPUTE = 16, KW_TMA = 16, KW_MMA = 17, KW_MMA_DK = 18, KW_PULL = 19;
+constexpr int DKDV_THREADS = (KW_COMPUTE + 4) * 32;   // 5 warps per scheduler: 96 registers each
 // Tail of the dK/dV kernel's shared memory: alignment slack, barriers, and two buffers of 256
 // per-query statistics (-lse * log2e for 128 queries, then -delta for the same 128).
-constexpr int DKDV_ALIGN_SLACK = 768, DKDV_BAR_BYTES = 192, DKDV_STAT_BYTES = 2 * 256 * 4;
+constexpr int DKDV_ALIGN_SLACK = 768, DKDV_BAR_BYTES = 224, DKDV_STAT_BYTES = 2 * 256 * 4;
 constexpr int DKDV_SMEM =
     2 * TILE_BYTES /*K,V*/ + (Q_STAGES + DO_STAGES) * TILE_BYTES + DKDV_ALIGN_SLACK + DKDV_BAR_BYTES + DKDV_STAT_BYTES;
+static_assert(DO_STAGES == 2, "the issuing warps use n & 1 as dO's stage");
 static_assert(DKDV_SMEM <= 227 * 1024, "dK/dV kernel shared memory");
 
 template <bool SPARSE>
@@ -213,16 +216,18 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* q_empty = bars + 4;     // [3]
   uint64_t* do_full = bars + 7;     // [2]
   uint64_t* do_empty = bars + 9;    // [2]
-  uint64_t* s_full = bars + 11;     // 1
-  uint64_t* dp_full = bars + 12;    // 1
-  uint64_t* p_ready = bars + 13;    // 1 (one arrival per compute warp)
-  uint64_t* ds_ready = bars + 14;   // 1 (one arrival per compute warp)
-  uint64_t* acc_done = bars + 15;   // 1
-  uint64_t* drain_bar = bars + 16;  // 1
-  uint64_t* stat_ready = bars + 17; // [2] (one arrival per publishing warp)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* s_full = bars + 11;     // [2] S^T of query half h is in TMEM
+  uint64_t* dp_full = bars + 13;    // [2]
+  uint64_t* p_ready = bars + 15;    // [2] (one arrival per compute warp of the half)
+  uint64_t* ds_ready = bars + 17;   // [2]
+  uint64_t* stat_full = bars + 19;  // [2] statistics of an item are in shared memory
+  uint64_t* stat_free = bars + 21;  // [2] (one arrival per compute warp)
+  uint64_t* acc_done = bars + 23;   // 1 (one commit per MMA warp)
+  uint64_t* drain_bar = bars + 24;  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* stats = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + DKDV_BAR_BYTES);  // [2][256]
+  int* item_qpos = reinterpret_cast<int*>(bars + 27);   // [2] position of the item's first query
+  float* stats = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + DKDV_BAR_BYTES);  // [2][-lse * log2e | -delta][128]
   if (smem - smem_raw > DKDV_ALIGN_SLACK) {  // same verdict in every thread
     if (threadIdx.x == 0) report(p.status, ZX_ERR_ARG, /*site=*/20, (int)(smem - smem_raw));
     return;
@@ -230,13 +235,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // Head-major: the CTAs in flight then share one or two heads' Q and dO tiles in L2 (measured 2 % faster than
-  // spreading them over all heads). Inside a head, early KV tiles (most work under a causal mask) run first.
-  int bid = blockIdx.x;
-  const int j = bid % p.n_kv_tiles;
-  bid /= p.n_kv_tiles;
-  const int b = bid % p.B;
-  const int hk = bid / p.B;
+  const WorkItem wi = work_item(blockIdx.x, p.n_kv_tiles, p.B * p.Hkv, p.kv_heads_per_group);
+  const int j = wi.tile;   // early KV tiles have the most work under a causal mask
+  const int b = wi.head / p.Hkv, hk = wi.head % p.Hkv;
   const int G = p.Hq / p.Hkv;
   const int kpos0 = kv_tile_pos(p, j);
 
@@ -248,16 +249,19 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     for (int s = 0; s < DO_STAGES; ++s) {
       mbar_init(&do_full[s], 1);
-      mbar_init(&do_empty[s], 1);
+      mbar_init(&do_empty[s], 2);   // one commit per MMA warp
     }
-    mbar_init(s_full, 1);
-    mbar_init(dp_full, 1);
-    mbar_init(p_ready, KW_COMPUTE);      // per-warp arrivals
-    mbar_init(ds_ready, KW_COMPUTE);
-    mbar_init(acc_done, 1);
-    mbar_init(drain_bar, 1);
-    mbar_init(&stat_ready[0], 8);
-    mbar_init(&stat_ready[1], 8);
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&s_full[h], 1);
+      mbar_init(&dp_full[h], 1);
+      mbar_init(&p_ready[h], KW_COMPUTE / 2);      // per-warp arrivals
+      mbar_init(&ds_ready[h], KW_COMPUTE / 2);
+      mbar_init(&stat_full[h], 1);
+      mbar_init(&stat_free[h], KW_COMPUTE);
+    }
+    mbar_init(acc_done, 2);
+    mbar_init(&drain_bar[0], 1);
+    mbar_init(&drain_bar[1], 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -280,9 +284,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (warp == KW_PULL) warp_pull_slice(p.pull_src, p.pull_dst, p.pull_nvec, lane);
 
-  if (n_items > 0 && warp < KW_PULL) {
+  if (n_items > 0 && warp != KW_PULL) {
     if (warp == KW_TMA) {
-      // ------------------------------- TMA producer -------------------------------
+      // ------------------------------- producer -----------------------------------
+      // Tiles through the TMA unit (lane 0), and what the compute warps need to know about each item: the position of
+      // its first query, -lse * log2e and -delta of its 128 queries. The compute warps so hold no walk state, no
+      // pointers and no prefetched values, which is what keeps them under 96 registers: a spilled register costs an
+      // L2 round trip here, since shared memory takes almost all of the L1.
       if (lane == 0) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmdO);
@@ -291,160 +299,150 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tma_load_4d(sK + HALF_BYTES, &tmK, kv_full, 64, hk, j * BT, b);
         tma_load_4d(sV, &tmV, kv_full, 0, hk, j * BT, b);
         tma_load_4d(sV + HALF_BYTES, &tmV, kv_full, 64, hk, j * BT, b);
-        uint32_t n = 0;
-        bool ok = true;
-        for (int g = 0; g < G && ok; ++g) {
-          const int hq = hk * G + g;
-          QWalk<SPARSE> w;
-          for (w.init(); w.next(p, kpos0);) {
-            const int t = w.t;
-            const int qs = n % Q_STAGES, ds = n % DO_STAGES;
-            if (!mbar_wait(&q_empty[qs], ((n / Q_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+      }
+      uint32_t n = 0;
+      bool ok = true;
+      for (int g = 0; g < G && ok; ++g) {
+        const int hq = hk * G + g;
+        const size_t row0 = ((size_t)b * p.Hq + hq) * p.Sq + lane;
+        QWalk<SPARSE> w;
+        for (w.init(); w.next(p, kpos0); ++n) {
+          const int t = w.t;
+          const int qs = n % Q_STAGES, ds = n % DO_STAGES;
+          float x[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            x[i] = __ldg(p.lse + row0 + (size_t)t * BT + 32 * i);
+            x[4 + i] = __ldg(p.delta + row0 + (size_t)t * BT + 32 * i);
+          }
+          if (!mbar_wait_w(&q_empty[qs], ((n / Q_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (lane == 0) {
             mbar_expect_tx(&q_full[qs], TILE_BYTES);
             tma_load_4d(sQ + qs * TILE_BYTES, &tmQ, &q_full[qs], 0, hq, t * BT, b);
             tma_load_4d(sQ + qs * TILE_BYTES + HALF_BYTES, &tmQ, &q_full[qs], 64, hq, t * BT, b);
-            if (!mbar_wait(&do_empty[ds], ((n / DO_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          }
+          if (!mbar_wait_w(&do_empty[ds], ((n / DO_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (lane == 0) {
             mbar_expect_tx(&do_full[ds], TILE_BYTES);
             tma_load_4d(sdO + ds * TILE_BYTES, &tmdO, &do_full[ds], 0, hq, t * BT, b);
             tma_load_4d(sdO + ds * TILE_BYTES + HALF_BYTES, &tmdO, &do_full[ds], 64, hq, t * BT, b);
-            ++n;
           }
-        }
-        if (!ok) {
-          report(p.status, ZX_ERR_TIMEOUT, /*site=*/21, (int)n);
-          const uint64_t t0 = globaltimer_ns();
-          while (globaltimer_ns() - t0 < 2000000ull) {
+          if (!mbar_wait_w(&stat_free[n & 1], ((n >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          float* st = stats + (n & 1) * 256 + lane;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            st[32 * i] = -LOG2E * x[i];
+            st[128 + 32 * i] = -x[4 + i];
           }
+          if (lane == 0) item_qpos[n & 1] = w.qpos0;
+          mbar_arrive_warp(&stat_full[n & 1]);
         }
       }
-    } else if (warp == KW_MMA) {
-      // ------------------------------- MMA issuer ---------------------------------
-      {  // all 32 lanes run this loop; the instructions themselves are issued by one elected lane
-        constexpr uint32_t idesc_kk = make_idesc(BT, BT, 1, 1, 0, 0);  // both operands K-major
-        constexpr uint32_t idesc_tm = make_idesc(BT, HD, 1, 1, 0, 1);  // A from TMEM, B MN-major
-        const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 384;
-        const uint64_t k_addr = base_kmajor(smem_u32(sK)), v_addr = base_kmajor(smem_u32(sV));
-        const uint64_t q_k0 = base_kmajor(smem_u32(sQ)), do_k0 = base_kmajor(smem_u32(sdO));
-        const uint64_t q_mn0 = base_mnmajor(smem_u32(sQ)), do_mn0 = base_mnmajor(smem_u32(sdO));
-        bool ok = mbar_wait_w(kv_full, 0, abort_flag);
-        ok = ok && mbar_wait_w(&q_full[0], 0, abort_flag);
-        ok = ok && mbar_wait_w(&do_full[0], 0, abort_flag);
-        tc_fence_after();
-        if (ok) {
-          umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_s, k_addr, q_k0, idesc_kk, 0u);
-          umma_commit_w(s_full);
-          umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_dp, v_addr, do_k0, idesc_kk, 0u);
-          umma_commit_w(dp_full);
+      if (!ok) {
+        if (lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/21, (int)n);
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) {
         }
-        int n = 0;
-        for (; n < n_items && ok; ++n) {
-          const int qs = n % Q_STAGES, ds = n % DO_STAGES;
-          const int qsn = (n + 1) % Q_STAGES, dsn = (n + 1) % DO_STAGES;
-          const bool has_next = n + 1 < n_items;
-          const uint64_t q_addr = desc_advance(q_mn0, (uint32_t)qs * TILE_BYTES);     // read transposed
-          const uint64_t do_addr = desc_advance(do_mn0, (uint32_t)ds * TILE_BYTES);   // read transposed
-          const uint64_t qn_addr = desc_advance(q_k0, (uint32_t)qsn * TILE_BYTES);
-          const uint64_t don_addr = desc_advance(do_k0, (uint32_t)dsn * TILE_BYTES);
-          // dV += P^T dO
-          if (!mbar_wait_w(p_ready, n & 1, abort_flag)) { ok = false; break; }
+      }
+    } else if (warp == KW_MMA || warp == KW_MMA_DK) {
+      // ------------------------------- MMA issuers --------------------------------
+      // Two issuing warps: one for S^T and dV (it owns the S^T / P^T columns and the dV accumulator), one for dP^T and
+      // dK. A wait costs such a warp some 270 clk even when its barrier completed long ago (a chain of dependent
+      // instructions that shares its scheduler with four compute warps), and only two MMAs are queued behind the one
+      // that runs, so one warp with all four products leaves the tensor core idle at each of its six waits per item
+      // (measured 4,200 clk per item against 2,480 of MMA time). With two, one issues while the other waits.
+      // All 32 lanes run the loops; the instructions themselves are issued by one elected lane.
+      const bool scores = warp == KW_MMA;
+      constexpr uint32_t idesc_kk = make_idesc(BT, BT / 2, 1, 1, 0, 0);  // both operands K-major, 64 queries
+      constexpr uint32_t idesc_tm = make_idesc(BT, HD, 1, 1, 0, 1);      // A from TMEM, B MN-major
+      // [S^T | dP^T] of both halves and the accumulator [dV | dK] of this warp
+      const uint32_t t_x = tmem_base + (scores ? 0 : 128), t_acc = tmem_base + (scores ? 256 : 384);
+      const uint64_t kv_addr = base_kmajor(smem_u32(scores ? sK : sV));
+      const uint64_t x_k0 = base_kmajor(smem_u32(scores ? sQ : sdO));      // B operand of the first product, as stored
+      const uint64_t x_mn0 = base_mnmajor(smem_u32(scores ? sdO : sQ));    // B operand of the second, read transposed
+      uint64_t* x_full = scores ? q_full : do_full;
+      uint64_t* out_full = scores ? s_full : dp_full;
+      uint64_t* in_ready = scores ? p_ready : ds_ready;
+      // first product of query half h: 64 rows of the tile are the B operand (HALF_Q bytes further down for h = 1)
+      auto first = [&](int h, int stage) {
+        umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_x + 64 * h, kv_addr, desc_advance(x_k0, (uint32_t)stage * TILE_BYTES + h * HALF_Q),
+                                             idesc_kk, 0u);
+        umma_commit_w(&out_full[h]);
+      };
+      // dV += P^T dO or dK += dS^T Q over the 64 queries of half h
+      auto second = [&](int h, int stage, uint32_t acc) {
+        umma_ts_k4_w<8, 32, 40>(t_acc, t_x + 64 * h, desc_advance(x_mn0, (uint32_t)stage * TILE_BYTES + h * HALF_Q), idesc_tm, acc);
+      };
+      bool ok = mbar_wait_w(kv_full, 0, abort_flag);
+      ok = ok && mbar_wait_w(&x_full[0], 0, abort_flag);
+      tc_fence_after();
+      if (ok) {
+        first(0, 0);
+        first(1, 0);
+        if (!scores) umma_commit_w(&do_empty[0]);   // dO(0) has served dP^T
+      }
+      int n = 0, qs = 0, qsn = 1 % Q_STAGES;        // stages of items n and n + 1, phase of the latter
+      uint32_t qphn = 0;
+      for (; n < n_items && ok; ++n) {
+        const int ds = n & 1, dsn = ds ^ 1;
+        const uint32_t dphn = ((n + 1) >> 1) & 1;
+        const bool has_next = n + 1 < n_items;
+        const int s_first = scores ? qsn : dsn, s_second = scores ? ds : qs;
+        if (has_next && !mbar_wait_w(&x_full[s_first], scores ? qphn : dphn, abort_flag)) { ok = false; break; }
+        for (int h = 0; h < 2; ++h) {
+          if (!mbar_wait_w(&in_ready[h], n & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          if (lane == 0) ZX_TRACE_DKDV(n, 8);
-          umma_ts_k8_w<8, 32, 40, 64, 72, 96, 104>(t_dv, t_s, do_addr, idesc_tm, n > 0 ? 1u : 0u);
-          umma_commit_w(&do_empty[ds]);   // dO(n) has now served dP^T(n) and dV(n)
-          if (lane == 0) ZX_TRACE_DKDV(n, 9);
-          if (has_next) {
-            if (!mbar_wait_w(&q_full[qsn], ((n + 1) / Q_STAGES) & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            if (lane == 0) ZX_TRACE_DKDV(n, 10);
-            umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_s, k_addr, qn_addr, idesc_kk, 0u);
-            umma_commit_w(s_full);
-            if (lane == 0) ZX_TRACE_DKDV(n, 15);
-          }
-          // dK += dS^T Q
-          if (!mbar_wait_w(ds_ready, n & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          if (lane == 0) ZX_TRACE_DKDV(n, 11);
-          umma_ts_k8_w<8, 32, 40, 64, 72, 96, 104>(t_dk, t_dp, q_addr, idesc_tm, n > 0 ? 1u : 0u);
-          umma_commit_w(&q_empty[qs]);    // Q(n) has now served S^T(n) and dK(n)
-          if (lane == 0) ZX_TRACE_DKDV(n, 12);
-          if (has_next) {
-            if (!mbar_wait_w(&do_full[dsn], ((n + 1) / DO_STAGES) & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            if (lane == 0) ZX_TRACE_DKDV(n, 13);
-            umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_dp, v_addr, don_addr, idesc_kk, 0u);
-            umma_commit_w(dp_full);
-          }
+          if (lane == 0) ZX_TRACE_DKDV(n, 8 + 2 * h + (scores ? 0 : 4));
+          second(h, s_second, (n > 0 || h > 0) ? 1u : 0u);
+          if (has_next) first(h, s_first);
+          if (lane == 0) ZX_TRACE_DKDV(n, 9 + 2 * h + (scores ? 0 : 4));
         }
-        if (ok) umma_commit_w(acc_done);
-        if (!ok) {
-          if (lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/22, n);
-          umma_commit_w(drain_bar);
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 50000000ull) {
-          }
+        if (!ok) break;
+        if (scores) {
+          umma_commit_w(&do_empty[ds]);                  // dV(n) has read dO(n)
+        } else {
+          umma_commit_w(&q_empty[qs]);                   // dK(n) has read Q(n); S^T(n) had long before
+          if (has_next) umma_commit_w(&do_empty[dsn]);   // dP^T(n+1) has read dO(n+1)
+        }
+        qs = qsn;
+        if (++qsn == Q_STAGES) { qsn = 0; qphn ^= 1u; }
+      }
+      if (ok) umma_commit_w(acc_done);
+      if (!ok) {
+        if (lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/22, n);
+        uint64_t* db = &drain_bar[scores ? 0 : 1];
+        umma_commit_w(db);
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(db, 0) && globaltimer_ns() - t0 < 50000000ull) {
         }
       }
     } else {
       // ------------------------------- compute warps ------------------------------
-      // Four column groups: group wg owns query columns [32 wg, 32 wg + 32) of every KV row.
+      // Four column groups: group wg owns query columns [32 wg, 32 wg + 32) of every KV row; groups 0, 1 are query
+      // half 0, groups 2, 3 half 1.
       const int wg = warp >> 2;
+      const int half = wg >> 1;
       const int lq = warp & 3;                 // TMEM lane quarter
       const int r = lq * 32 + lane;            // KV row of this thread == TMEM lane
       const int col0 = wg * 32;
       const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
       const uint32_t t_s = tmem_base + lane_base + col0, t_dp = tmem_base + lane_base + 128 + col0;
       const int my_kpos = kpos0 + r;
-      uint32_t n = 0;
+      int n = 0;
       bool ok = true;
-      // Per-query statistics reach the math through shared memory, one item ahead: thread i of
-      // the 256 fetches one value of the NEXT item (-lse * log2e for i < 128, -delta otherwise)
-      // at the top of an iteration and publishes it at the bottom, so no global-load latency
-      // sits between a TMEM read and its use. Buffer (n + 1) & 1 was last read in iteration
-      // n - 1, and every thread finished that before dP^T(n) could be issued.
-      const int ct = threadIdx.x;  // 0..255
-      // this thread's statistic of item (g, t): -lse * log2e of query ct for ct < 128, else -delta of query ct - 128
-      const float* stat_src = (ct < BT ? p.lse : p.delta) + ((size_t)b * p.Hq + (size_t)hk * G) * p.Sq + (ct & (BT - 1));
-      const float stat_mul = ct < BT ? -LOG2E : -1.f;
-      auto stat_fetch = [&](int g, int t) -> float {
-        return stat_mul * __ldg(stat_src + (size_t)g * p.Sq + (size_t)t * BT);
-      };
-      QWalk<SPARSE> walk;
-      auto next_item = [&](int& g) -> bool {   // advances walk (and g when a head's tiles are exhausted)
-        for (;;) {
-          if (walk.next(p, kpos0)) return true;
-          walk.init();
-          if (++g >= G) return false;
-        }
-      };
-      int g = 0;
-      walk.init();
-      bool have = next_item(g);
-      int t = walk.t, qpos0 = walk.qpos0;
-      if (have && ct < 256) {
-        stats[ct] = stat_fetch(g, t);
-        mbar_arrive_warp(&stat_ready[0]);
-      }
-      while (have) {
-        int gn = g;
-        const bool have_next = next_item(gn);
-        const int tn = walk.t, qposn = walk.qpos0;
-        float pre = 0.f;
-        if (have_next && ct < 256) pre = stat_fetch(gn, tn);
-        const float* st = stats + (n & 1) * 256;
-        if (!wait_warp(&stat_ready[n & 1], (n >> 1) & 1, abort_flag)) { ok = false; break; }
-        ZX_TRACE_W(n, 7);
-        if (!wait_warp(s_full, n & 1, abort_flag)) { ok = false; break; }
+      for (; n < n_items; ++n) {
+        const float* st = stats + (n & 1) * 256 + col0;
+        if (!wait_warp(&stat_full[n & 1], (n >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!wait_warp(&s_full[half], n & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 0);
-        ZX_TRACE_W(n, 0);
+        if (threadIdx.x == 256) ZX_TRACE_DKDV(n, 4);
         uint32_t sr[32];
         tmem_ld_32x32b_x32(t_s, sr);
         tmem_wait_ld();
-        ZX_TRACE_W(n, 1);
-        const bool diag = p.causal && (kpos0 + BT - 1 > qpos0);
-        const int qp = qpos0 + col0;   // column c is query qp + c; it sees this key iff my_kpos <= qp + c
+        const int qpos0 = item_qpos[n & 1];
         const float2 sl2 = make_float2(p.scale_log2, p.scale_log2);
-        const float4* nl4 = reinterpret_cast<const float4*>(st + col0);   // uniform address: broadcast reads
+        const float4* nl4 = reinterpret_cast<const float4*>(st);   // uniform address: broadcast reads
         static_for<8>([&](auto idx4) {
           constexpr int c4 = decltype(idx4)::value;
           const float4 nl = nl4[c4];
@@ -458,12 +456,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             sr[2 * c + 1] = __float_as_uint(e.y);
           });
         });
-        if (diag) {   // only tiles on the diagonal pay for the per-element mask
+        if (p.causal && kpos0 + BT - 1 > qpos0) {   // only tiles on the diagonal pay for the per-element mask
+          const int seen = my_kpos - qpos0 - col0;   // this key is visible to columns c >= seen
 #pragma unroll
           for (int c = 0; c < 32; ++c)
-            if (my_kpos > qp + c) sr[c] = 0u;
+            if (c < seen) sr[c] = 0u;
         }
-        ZX_TRACE_W(n, 2);
         {
           // bf16 P^T of this group goes over the first 16 of the 32 columns this thread just read
           uint32_t pk[16];
@@ -472,21 +470,20 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tmem_st_32x32b_x16(t_s, pk);
         }
         tmem_wait_st();
-        if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 2);
-        ZX_TRACE_W(n, 3);
+        if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 1);
+        if (threadIdx.x == 256) ZX_TRACE_DKDV(n, 5);
         tc_fence_before();
-        mbar_arrive_warp(p_ready);
-        if (!wait_warp(dp_full, n & 1, abort_flag)) { ok = false; break; }
+        mbar_arrive_warp(&p_ready[half]);
+        if (!wait_warp(&dp_full[half], n & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 3);
-        ZX_TRACE_W(n, 4);
+        if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 2);
+        if (threadIdx.x == 256) ZX_TRACE_DKDV(n, 6);
         uint32_t dp[32];
         tmem_ld_32x32b_x32(t_dp, dp);
         tmem_wait_ld();
-        ZX_TRACE_W(n, 5);
         {
           uint32_t dsp[16];
-          const float4* nd4 = reinterpret_cast<const float4*>(st + BT + col0);
+          const float4* nd4 = reinterpret_cast<const float4*>(st + BT);
 #pragma unroll
           for (int e4 = 0; e4 < 8; ++e4) {
             const float4 nd = nd4[e4];
@@ -502,19 +499,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tmem_st_32x32b_x16(t_dp, dsp);
         }
         tmem_wait_st();
-        if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 5);
-        ZX_TRACE_W(n, 6);
+        if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 3);
         tc_fence_before();
-        mbar_arrive_warp(ds_ready);
-        if (have_next && ct < 256) {
-          stats[((n + 1) & 1) * 256 + ct] = pre;
-          mbar_arrive_warp(&stat_ready[(n + 1) & 1]);
-        }
-        g = gn;
-        t = tn;
-        qpos0 = qposn;
-        have = have_next;
-        ++n;
+        mbar_arrive_warp(&ds_ready[half]);
+        if (lane == 0) mbar_arrive(&stat_free[n & 1]);
       }
       // epilogue: add dV and scale * dK into the (possibly remote) fp32 accumulators; each
       // column group drains its 32 columns of both accumulators
@@ -591,12 +579,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // Head-major, late Q tiles (most work) first inside a head: the CTAs in flight stream the same K and V.
-  int bid = blockIdx.x;
-  const int t = p.n_q_tiles - 1 - bid % p.n_q_tiles;
-  bid /= p.n_q_tiles;
-  const int b = bid % p.B;
-  const int hq = bid / p.B;
+  const WorkItem wi = work_item(blockIdx.x, p.n_q_tiles, p.B * p.Hq, p.q_heads_per_group);
+  const int t = p.n_q_tiles - 1 - wi.tile;   // late Q tiles have the most work under a causal mask
+  const int b = wi.head / p.Hq, hq = wi.head % p.Hq;
   const int hk = hq / (p.Hq / p.Hkv);
   const int qpos0 = q_tile_pos(p, t);
 
@@ -910,6 +895,9 @@ void launch_attn_bwd(const AttnBwdArgs& a) {
     set_smem(attn_bwd_dq_kernel<true>, DQ_SMEM, "attn_bwd_dq (windowed)");
     configured = true;
   }
+  const bool uniform = !a.mask.causal && a.mask.window_blocks == 0;
+  p.kv_heads_per_group = heads_per_group(p.n_q_tiles, a.B * a.Hkv, uniform, a.mask.window_blocks > 0);
+  p.q_heads_per_group = heads_per_group(p.n_kv_tiles, a.B * a.Hq, uniform, false);
   const unsigned grid_kv = p.n_kv_tiles * a.B * a.Hkv, grid_q = p.n_q_tiles * a.B * a.Hq;
   if (p.window_blocks > 0) {
     attn_bwd_dkdv_kernel<true><<<grid_kv, DKDV_THREADS, DKDV_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, p);

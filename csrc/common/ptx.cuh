@@ -344,10 +344,11 @@ __device__ __forceinline__ void umma_ts_k8_mnmajor_w(uint32_t d_tmem, uint32_t a
                                                      uint32_t acc_first) {
   umma_ts_k8_w<8, 16, 24, 32, 40, 48, 56>(d_tmem, a_tmem, b_desc, idesc, acc_first);
 }
-// Half of the above: four MMAs (K = 4 x 16 = 64), so that P V can start on the first 64 probabilities of a
-// row block while the softmax warps still work on the other 64.
-__device__ __forceinline__ void umma_ts_k4_mnmajor_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                     uint32_t acc_first) {
+// Half of the above: four MMAs (K = 4 x 16 = 64), so that a product can start on 64 of the 128 inner rows while the
+// other 64 are still being computed. A1..A3 as above.
+template <int A1, int A2, int A3>
+__device__ __forceinline__ void umma_ts_k4_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t acc_first) {
   asm volatile(
       "{\n\t"
       ".reg .pred e, p, t;\n\t"
@@ -357,14 +358,50 @@ __device__ __forceinline__ void umma_ts_k4_mnmajor_w(uint32_t d_tmem, uint32_t a
       "setp.ne.b32 p, %4, 0;\n\t"
       "setp.eq.b32 t, %3, %3;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "add.u32 ta, %1, 8;\n\t add.s64 b, %2, 128;\n\t"
+      "add.u32 ta, %1, %5;\n\t add.s64 b, %2, 128;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
-      "add.u32 ta, %1, 16;\n\t add.s64 b, %2, 256;\n\t"
+      "add.u32 ta, %1, %6;\n\t add.s64 b, %2, 256;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
-      "add.u32 ta, %1, 24;\n\t add.s64 b, %2, 384;\n\t"
+      "add.u32 ta, %1, %7;\n\t add.s64 b, %2, 384;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
       "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc_first)
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc_first), "n"(A1), "n"(A2), "n"(A3)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_k4_mnmajor_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                                     uint32_t acc_first) {
+  umma_ts_k4_w<8, 16, 24>(d_tmem, a_tmem, b_desc, idesc, acc_first);
+}
+// A (M x 128 bf16, 64 columns) read from TMEM, B K-major in shared memory as two 64-element halves.
+template <int HALF16>
+__device__ __forceinline__ void umma_ts_k8_kmajor_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                                    uint32_t acc_first) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e, p, t;\n\t"
+      ".reg .b32 ta;\n\t"
+      ".reg .b64 b;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.eq.b32 t, %3, %3;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "add.u32 ta, %1, 8;\n\t add.s64 b, %2, 2;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "add.u32 ta, %1, 16;\n\t add.s64 b, %2, 4;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "add.u32 ta, %1, 24;\n\t add.s64 b, %2, 6;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "add.u32 ta, %1, 32;\n\t add.s64 b, %2, %5;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "add.u32 ta, %1, 40;\n\t add.s64 b, %2, %6;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "add.u32 ta, %1, 48;\n\t add.s64 b, %2, %7;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "add.u32 ta, %1, 56;\n\t add.s64 b, %2, %8;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], b, %3, t;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc_first), "n"(HALF16), "n"(HALF16 + 2), "n"(HALF16 + 4),
+      "n"(HALF16 + 6)
       : "memory");
 }
 // Warp-uniform bounded wait: every lane polls, the verdict is shared.
