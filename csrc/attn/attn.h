@@ -61,9 +61,11 @@ struct AttnBwdArgs {
   const void* d_o = nullptr;  // [B, Sq, Hq, 128]
   const float* lse = nullptr; // [B, Hq, Sq]
   float* delta = nullptr;     // [B, Hq, Sq] scratch: rowsum(dO * O), written by the pre-pass
-  float* dq = nullptr;        // [B, Sq, Hq, 128] fp32, written (or accumulated when dq_accumulate)
-  float* dk = nullptr;        // [B, Skv, Hkv, 128] fp32, red.add target, caller zeroes (may be a peer's buffer)
-  float* dv = nullptr;        // [B, Skv, Hkv, 128] fp32, red.add target, caller zeroes (may be a peer's buffer)
+  void* dq = nullptr;         // [B, Sq, Hq, 128] fp32, written (or accumulated when dq_accumulate)
+  void* dk = nullptr;         // [B, Skv, Hkv, 128] fp32, red.add target, caller zeroes (may be a peer's buffer)
+  void* dv = nullptr;         // [B, Skv, Hkv, 128] fp32, red.add target, caller zeroes (may be a peer's buffer)
+  int kv_overwrite = 0;       // write dk and dv instead of adding to them (every key tile of this call, seen or not)
+  int out_bf16 = 0;           // dq, dk and dv are bf16 (each rounded once from fp32); written, never added to
   int B = 1, Hq = 0, Hkv = 0, Sq = 0, Skv = 0;
   int64_t q_tok_stride = 0, k_tok_stride = 0, v_tok_stride = 0;
   float scale = 0.f;
@@ -71,8 +73,8 @@ struct AttnBwdArgs {
   AttnLayout q_layout, kv_layout;
   int compute_delta = 1;  // run the delta pre-pass (once per backward; later ring steps reuse it)
   int dq_accumulate = 0;  // add to the dq already present instead of overwriting it (ring step > 0)
-  // Optional in-kernel timeline of the dQ kernel's first CTA: 64 iterations x 16 slots of SM clock
-  // stamps (slots 0-5: compute thread 0 after each phase, 8-10: MMA warp). Null: no tracing.
+  // Optional in-kernel timeline of the dK/dV kernel's first CTA (builds with -DZX_BWD_TRACE): from element 1024 on,
+  // 64 iterations x 16 slots of SM clock stamps (0-3 first compute warp, 4-6 first warp of the second half). Null: none.
   long long* trace = nullptr;
   const void* pull_src = nullptr;  // same fused peer pull as in the forward (done by the dK/dV kernel)
   void* pull_dst = nullptr;

@@ -7,12 +7,20 @@
 //               lanes, which is exactly the A operand of dV += P^T dO and dK += dS^T Q.
 //               The result is added to fp32 dK/dV with red.add (system scope): the destination may
 //               be a peer GPU's buffer, which is how a ring step returns gradients to the KV owner.
+//               (kv_overwrite: written instead, in fp32 or bf16, when nothing else adds to it.)
 //  dq kernel    one CTA per (Q tile, query head): S = Q K^T, dP = dO V^T, dQ += dS K with dS fed
 //               from TMEM; deterministic, no atomics.
 //
-// In both kernels the MMA stream is staggered (S of the next tile is issued while the compute
-// warps still turn dP into dS), so exponentials and tensor work overlap with a single softmax
-// warpgroup. All waits are bounded.
+// Both kernels cut a 128 x 128 item into two halves of 64 columns (queries / keys), each with eight compute warps and
+// its own score and dP columns in TMEM, and issue from two warps. A half is a dependency cycle scores -> exponentials
+// -> product -> next scores; with a single 128-wide cycle the tensor core waited for the exponentials and the
+// exponentials for the tensor core (3,620 clk per item in the dK/dV kernel against 2,048 of MMA time), the two halves
+// run in opposite phases (2,830 clk). The price is 64-wide products with both operands in shared memory, which run at
+// 48 clk per step instead of 32 (6 KB at 128 B/clk): 2,480 clk of MMA time per item in the dK/dV kernel, whose TMEM is
+// full. The dQ kernel has room for Q and dO in TMEM and pays nothing (2,110 -> 1,740 clk per item, MMA time 1,536).
+// Kernel times, 32 heads over 8 KV heads, causal (before -> now): dK/dV 1,140 -> 816 us at 8,192 tokens, 16.2 -> 13.6 ms
+// at 32,768; dQ 709 -> 635 us and 11.0 -> 9.5 ms (the GPU runs at its power cap at 32,768, 1.5 GHz).
+// All waits are bounded.
 #include "../common/ptx.cuh"
 #include "../common/device_once.h"
 #include "../common/tma_host.h"
@@ -31,9 +39,6 @@ constexpr int BT = 128;                    // tile edge in tokens (both Q and KV
 constexpr int TILE_BYTES = BT * HD * 2;    // 32 KB
 constexpr int HALF_BYTES = TILE_BYTES / 2; // one 64-wide d chunk
 constexpr int HALF_Q = 64 * 128;           // 64 rows of a d chunk: start of a tile's second half of tokens
-constexpr int NUM_THREADS = 352;           // dQ kernel: 8 compute warps (two warpgroups) + TMA warp + two MMA warps
-constexpr int W_TMA = 8, W_MMA = 9, W_MMA_DQ = 10;   // dQ kernel roles (the dK/dV kernel has its own, below)
-constexpr int N_COMPUTE = 256;             // compute threads
 constexpr int TMEM_COLS = 512;
 constexpr float LOG2E = 1.4426950408889634f;
 // Every BWD_POLY_EVERY-th pair of exponentials can be evaluated as a polynomial on the FMA pipe instead of the
@@ -55,7 +60,7 @@ struct BwdParams {
   float scale, scale_log2;
   int causal, window_blocks, global_every;
   int n_q_tiles, n_kv_tiles;
-  int q_tiles_per_chunk, kv_tiles_per_chunk;
+  int q_tiles_per_chunk, kv_tiles_per_chunk, n_q_chunks, n_kv_chunks;
   int kv_heads_per_group, q_heads_per_group;   // block order, see work_item
   int q_chunk_pos[kAttnMaxChunks];
   int kv_chunk_pos[kAttnMaxChunks];
@@ -64,7 +69,7 @@ struct BwdParams {
   float* dq;
   float* dk;
   float* dv;
-  int dq_accumulate;
+  int dq_accumulate, kv_overwrite, out_bf16;
   const uint4* pull_src;
   uint4* pull_dst;
   size_t pull_nvec;
@@ -72,20 +77,15 @@ struct BwdParams {
   Status* status;
 };
 
-// Clock stamps of pipeline events into the caller's trace buffer (first CTA of each kernel). Compiled in only
+// Clock stamps of pipeline events into the caller's trace buffer (first CTA of the dK/dV kernel). Compiled in only
 // with -DZX_BWD_TRACE: the stamps cost issue slots in loops that are bound by instruction issue.
 #ifdef ZX_BWD_TRACE
 #define ZX_TRACE_DKDV(iter, slot)                                                     \
   do {                                                                                \
     if (p.trace != nullptr && blockIdx.x == 0 && (iter) < 64) p.trace[1024 + (iter) * 16 + (slot)] = clock64(); \
   } while (0)
-#define ZX_TRACE(iter, slot)                                                          \
-  do {                                                                                \
-    if (p.trace != nullptr && blockIdx.x == 0 && (iter) < 64) p.trace[(iter) * 16 + (slot)] = clock64(); \
-  } while (0)
 #else
 #define ZX_TRACE_DKDV(iter, slot) do { } while (0)
-#define ZX_TRACE(iter, slot) do { } while (0)
 #endif
 
 __device__ __forceinline__ int q_tile_pos(const BwdParams& p, int t) {
@@ -94,13 +94,19 @@ __device__ __forceinline__ int q_tile_pos(const BwdParams& p, int t) {
 __device__ __forceinline__ int kv_tile_pos(const BwdParams& p, int j) {
   return p.kv_chunk_pos[j / p.kv_tiles_per_chunk] + (j % p.kv_tiles_per_chunk) * BT;
 }
-// The Q tiles that may attend the KV tile at position kpos0, in order. The backward kernels are bound by
-// instruction issue, and every role of a CTA walks this sequence once per item, so the dense instantiation
-// keeps the position incrementally (no division, no search); windowed masks use the jumping search.
+// The Q tiles that may attend the KV tile at position kpos0, in order. Positions grow with the tile index inside a
+// chunk, so without a window the visible tiles of a chunk are its last ones and the walk starts at the first of them
+// (a walk that tests every tile from 0 costs a late KV tile several microseconds before its first load, in every
+// role); windowed masks use the jumping search. `count` is the number of tiles `next` will return.
 template <bool SPARSE>
 struct QWalk {
-  int t, qpos0, in_chunk, c;
-  __device__ __forceinline__ void init() { t = -1; qpos0 = 0; in_chunk = 0; c = 0; }
+  int t, qpos0, left, c;
+  __device__ __forceinline__ void init() { t = -1; qpos0 = 0; left = 0; c = -1; }
+  // first visible tile of chunk c
+  static __device__ __forceinline__ int first_in_chunk(const BwdParams& p, int c, int kpos0) {
+    const int d = p.causal ? (kpos0 - p.q_chunk_pos[c]) / BT : 0;
+    return d < 0 ? 0 : (d < p.q_tiles_per_chunk ? d : p.q_tiles_per_chunk);
+  }
   __device__ __forceinline__ bool next(const BwdParams& p, int kpos0) {
     if constexpr (SPARSE) {
       t = next_q_tile(p, kpos0, t + 1);
@@ -108,21 +114,40 @@ struct QWalk {
       qpos0 = q_tile_pos(p, t);
       return true;
     } else {
-      for (;;) {
-        if (++t >= p.n_q_tiles) return false;
-        if (in_chunk == p.q_tiles_per_chunk) { ++c; in_chunk = 0; }
-        qpos0 = p.q_chunk_pos[c] + in_chunk * BT;
-        ++in_chunk;
-        if (!(p.causal && kpos0 > qpos0)) return true;
+      ++t;
+      qpos0 += BT;
+      while (left == 0) {
+        if (++c >= p.n_q_chunks) return false;
+        const int i = first_in_chunk(p, c, kpos0);
+        left = p.q_tiles_per_chunk - i;
+        t = c * p.q_tiles_per_chunk + i;
+        qpos0 = p.q_chunk_pos[c] + i * BT;
       }
+      --left;
+      return true;
     }
   }
+  static __device__ __forceinline__ int count(const BwdParams& p, int kpos0) {
+    int n = 0;
+    if constexpr (SPARSE) {
+      QWalk w;
+      for (w.init(); w.next(p, kpos0);) ++n;
+    } else {
+      for (int c = 0; c < p.n_q_chunks; ++c) n += p.q_tiles_per_chunk - first_in_chunk(p, c, kpos0);
+    }
+    return n;
+  }
 };
-// The KV tiles the Q tile at position qpos0 may attend, in order.
+// The KV tiles the Q tile at position qpos0 may attend, in order: without a window the first ones of each chunk.
 template <bool SPARSE>
 struct KvWalk {
-  int j, kpos0, in_chunk, c;
-  __device__ __forceinline__ void init() { j = -1; kpos0 = 0; in_chunk = 0; c = 0; }
+  int j, kpos0, left, c;
+  __device__ __forceinline__ void init() { j = -1; kpos0 = 0; left = 0; c = -1; }
+  static __device__ __forceinline__ int in_chunk(const BwdParams& p, int c, int qpos0) {
+    if (!p.causal) return p.kv_tiles_per_chunk;
+    const int d = qpos0 - p.kv_chunk_pos[c];
+    return d < 0 ? 0 : (d / BT + 1 < p.kv_tiles_per_chunk ? d / BT + 1 : p.kv_tiles_per_chunk);
+  }
   __device__ __forceinline__ bool next(const BwdParams& p, int qpos0) {
     if constexpr (SPARSE) {
       j = next_kv_tile(p, qpos0, j + 1);
@@ -130,14 +155,27 @@ struct KvWalk {
       kpos0 = kv_tile_pos(p, j);
       return true;
     } else {
-      for (;;) {
-        if (++j >= p.n_kv_tiles) return false;
-        if (in_chunk == p.kv_tiles_per_chunk) { ++c; in_chunk = 0; }
-        kpos0 = p.kv_chunk_pos[c] + in_chunk * BT;
-        ++in_chunk;
-        if (!(p.causal && kpos0 > qpos0)) return true;
+      ++j;
+      kpos0 += BT;
+      while (left == 0) {
+        if (++c >= p.n_kv_chunks) return false;
+        left = in_chunk(p, c, qpos0);
+        j = c * p.kv_tiles_per_chunk;
+        kpos0 = p.kv_chunk_pos[c];
       }
+      --left;
+      return true;
     }
+  }
+  static __device__ __forceinline__ int count(const BwdParams& p, int qpos0) {
+    int n = 0;
+    if constexpr (SPARSE) {
+      KvWalk w;
+      for (w.init(); w.next(p, qpos0);) ++n;
+    } else {
+      for (int c = 0; c < p.n_kv_chunks; ++c) n += in_chunk(p, c, qpos0);
+    }
+    return n;
   }
 };
 
@@ -151,6 +189,37 @@ __device__ __forceinline__ void red_add_v4_sys(float* addr, float a, float b, fl
                : "memory");
 }
 
+// One warp's 32 rows x 32 columns of an accumulator (row = lane) into a slab of shared memory and from there to global
+// memory through the TMA unit, which writes whole lines; rows are swizzled so that the 16-byte writes of eight lanes
+// fall into different banks. (Thread-per-row stores, 16 bytes of 32 rows per instruction, took 4 to 6 us at the end of
+// every block.) The caller waits for the store before the block ends.
+constexpr int SLAB_BYTES = 32 * 128;
+__device__ __forceinline__ void store_slab(const CUtensorMap* m, uint8_t* slab, const uint32_t* a, float scale, int bf16,
+                                           int lane, int col, int head, int row, int batch) {
+  if (bf16) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        w[e] = pack_bf16x2(__uint_as_float(a[8 * c + 2 * e]) * scale, __uint_as_float(a[8 * c + 2 * e + 1]) * scale);
+      *reinterpret_cast<uint4*>(slab + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      *reinterpret_cast<float4*>(slab + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+          make_float4(__uint_as_float(a[4 * c]) * scale, __uint_as_float(a[4 * c + 1]) * scale,
+                      __uint_as_float(a[4 * c + 2]) * scale, __uint_as_float(a[4 * c + 3]) * scale);
+  }
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_4d(m, slab, col, head, row, batch);
+    tma_store_commit();
+  }
+}
+
 // Base descriptors of a [128 x 128] bf16 tile (built once per tile address) ...
 __device__ __forceinline__ uint64_t base_kmajor(uint32_t tile_addr) { return make_smem_desc_sw128(tile_addr, 16, 1024); }
 __device__ __forceinline__ uint64_t base_mnmajor(uint32_t tile_addr) {
@@ -159,24 +228,44 @@ __device__ __forceinline__ uint64_t base_mnmajor(uint32_t tile_addr) {
 // ------------------------------------------------------------------------------------------
 // delta[b, h, s] = sum_d dO * O
 // ------------------------------------------------------------------------------------------
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  float* __restrict__ delta, int B, int S, int H) {
-  const int warps_per_block = blockDim.x >> 5;
-  const size_t row = (size_t)blockIdx.x * warps_per_block + (threadIdx.x >> 5);  // (b, s, h)
-  const int lane = threadIdx.x & 31;
-  if (row >= (size_t)B * S * H) return;
-  const uint2 a = reinterpret_cast<const uint2*>(o + row * HD)[lane];
-  const uint2 g = reinterpret_cast<const uint2*>(d_o + row * HD)[lane];
-  const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), g0 = unpack_bf16x2(g.x), g1 = unpack_bf16x2(g.y);
-  float acc = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y;
+// Bound by memory: one warp takes eight consecutive tokens of one head (two 256-byte rows per load instruction, all
+// eight loads of a lane in flight, eight neighbouring results per store).
+constexpr int DELTA_TOKENS = 8;
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
+                                                         const __nv_bfloat16* __restrict__ d_o,
+                                                         float* __restrict__ delta, int S, int H, int n_groups) {
+  const int group = blockIdx.x * 8 + (threadIdx.x >> 5);   // (b, s / 8, h)
+  if (group >= n_groups) return;
+  const int lane = threadIdx.x & 31, sub = lane >> 4;
+  const int h = group % H, bs = group / H;   // bs: eighth of a token row over all batches (S is a multiple of 128)
+  const size_t row0 = ((size_t)bs * DELTA_TOKENS + sub) * H + h;
+  uint4 a[4], g[4];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) {
-    const int h = (int)(row % H);
-    const size_t bs = row / H;
-    const int s = (int)(bs % S);
-    const int b = (int)(bs / S);
-    delta[((size_t)b * H + h) * S + s] = acc;
+  for (int i = 0; i < 4; ++i) {
+    const size_t off = (row0 + (size_t)2 * i * H) * (HD / 8) + (lane & 15);
+    a[i] = __ldg(reinterpret_cast<const uint4*>(o) + off);
+    g[i] = __ldg(reinterpret_cast<const uint4*>(d_o) + off);
+  }
+  float out = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = unpack_bf16x2(aw[e]), y = unpack_bf16x2(gw[e]);
+      acc += x.x * y.x + x.y * y.y;
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    // token 2 i + sub of the group: lanes 0..7 end up with one token each
+    const float other = __shfl_xor_sync(0xffffffffu, acc, 16);
+    if ((lane >> 1) == i) out = (lane & 1) == sub ? acc : other;
+  }
+  if (lane < DELTA_TOKENS) {
+    const int per_batch = S / DELTA_TOKENS;
+    const int b = bs / per_batch, s = (bs % per_batch) * DELTA_TOKENS + lane;
+    delta[((size_t)b * H + h) * S + s] = out;
   }
 }
 
@@ -203,7 +292,8 @@ static_assert(DKDV_SMEM <= 227 * 1024, "dK/dV kernel shared memory");
 template <bool SPARSE>
 __global__ void __launch_bounds__(DKDV_THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
-                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdParams p) {
+                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                     const __grid_constant__ CUtensorMap tmGK, const __grid_constant__ CUtensorMap tmGV, BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
@@ -249,7 +339,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     for (int s = 0; s < DO_STAGES; ++s) {
       mbar_init(&do_full[s], 1);
-      mbar_init(&do_empty[s], 2);   // one commit per MMA warp
+      mbar_init(&do_empty[s], 1);
     }
     for (int h = 0; h < 2; ++h) {
       mbar_init(&s_full[h], 1);
@@ -275,12 +365,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
 
   // number of (head, q tile) items this CTA processes: identical in every role
-  int n_items = 0;
-  {
-    QWalk<SPARSE> w;
-    for (w.init(); w.next(p, kpos0);) ++n_items;
-  }
-  n_items *= G;
+  const int n_items = G * QWalk<SPARSE>::count(p, kpos0);
 
   if (warp == KW_PULL) warp_pull_slice(p.pull_src, p.pull_dst, p.pull_nvec, lane);
 
@@ -379,7 +464,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (ok) {
         first(0, 0);
         first(1, 0);
-        if (!scores) umma_commit_w(&do_empty[0]);   // dO(0) has served dP^T
       }
       int n = 0, qs = 0, qsn = 1 % Q_STAGES;        // stages of items n and n + 1, phase of the latter
       uint32_t qphn = 0;
@@ -388,22 +472,15 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint32_t dphn = ((n + 1) >> 1) & 1;
         const bool has_next = n + 1 < n_items;
         const int s_first = scores ? qsn : dsn, s_second = scores ? ds : qs;
-        if (has_next && !mbar_wait_w(&x_full[s_first], scores ? qphn : dphn, abort_flag)) { ok = false; break; }
         for (int h = 0; h < 2; ++h) {
-          if (!mbar_wait_w(&in_ready[h], n & 1, abort_flag)) { ok = false; break; }
+          const bool got = h == 0 && has_next ? mbar_wait2_w(&in_ready[0], n & 1, &x_full[s_first], scores ? qphn : dphn, abort_flag)
+                                              : mbar_wait_w(&in_ready[h], n & 1, abort_flag);
+          if (!got) { ok = false; break; }
           tc_fence_after();
-          if (lane == 0) ZX_TRACE_DKDV(n, 8 + 2 * h + (scores ? 0 : 4));
           second(h, s_second, (n > 0 || h > 0) ? 1u : 0u);
           if (has_next) first(h, s_first);
-          if (lane == 0) ZX_TRACE_DKDV(n, 9 + 2 * h + (scores ? 0 : 4));
         }
         if (!ok) break;
-        if (scores) {
-          umma_commit_w(&do_empty[ds]);                  // dV(n) has read dO(n)
-        } else {
-          umma_commit_w(&q_empty[qs]);                   // dK(n) has read Q(n); S^T(n) had long before
-          if (has_next) umma_commit_w(&do_empty[dsn]);   // dP^T(n+1) has read dO(n+1)
-        }
         qs = qsn;
         if (++qsn == Q_STAGES) { qsn = 0; qphn ^= 1u; }
       }
@@ -429,11 +506,15 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t t_s = tmem_base + lane_base + col0, t_dp = tmem_base + lane_base + 128 + col0;
       const int my_kpos = kpos0 + r;
       int n = 0;
+      int qs_prev = Q_STAGES - 1;   // stage of item n - 1
       bool ok = true;
       for (; n < n_items; ++n) {
         const float* st = stats + (n & 1) * 256 + col0;
         if (!wait_warp(&stat_full[n & 1], (n >> 1) & 1, abort_flag)) { ok = false; break; }
         if (!wait_warp(&s_full[half], n & 1, abort_flag)) { ok = false; break; }
+        // Stages are handed back here and not by commits of the issuing warps, whose queue they would fill: S^T of half
+        // 1 was issued after dV(n-1), so its arrival says that dO(n-1) has been read (and dP^T(n-1) long before) ...
+        if (threadIdx.x == 256 && n > 0) mbar_arrive(&do_empty[(n - 1) % DO_STAGES]);
         tc_fence_after();
         if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 0);
         if (threadIdx.x == 256) ZX_TRACE_DKDV(n, 4);
@@ -475,6 +556,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tc_fence_before();
         mbar_arrive_warp(&p_ready[half]);
         if (!wait_warp(&dp_full[half], n & 1, abort_flag)) { ok = false; break; }
+        // ... and dP^T of half 1 after dK(n-1), so Q(n-1) has been read
+        if (threadIdx.x == 256) {
+          if (n > 0) mbar_arrive(&q_empty[qs_prev]);
+          qs_prev = qs_prev + 1 == Q_STAGES ? 0 : qs_prev + 1;
+        }
         tc_fence_after();
         if (threadIdx.x == 0) ZX_TRACE_DKDV(n, 2);
         if (threadIdx.x == 256) ZX_TRACE_DKDV(n, 6);
@@ -504,11 +590,23 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         mbar_arrive_warp(&ds_ready[half]);
         if (lane == 0) mbar_arrive(&stat_free[n & 1]);
       }
-      // epilogue: add dV and scale * dK into the (possibly remote) fp32 accumulators; each
-      // column group drains its 32 columns of both accumulators
+      // epilogue: dV and scale * dK, each column group its 32 columns of both accumulators. Written through shared
+      // memory (the stages of Q and dO are free once every MMA has finished), or added into the (possibly remote) fp32
+      // accumulators.
       if (ok) ok = wait_warp(acc_done, 0, abort_flag);
       tc_fence_after();
-      if (ok && ZX_IN_BOUNDS(p.status, j * BT + r, p.Skv, 24)) {
+      const bool row_ok = ok && ZX_IN_BOUNDS(p.status, j * BT + r, p.Skv, 24);
+      if (p.kv_overwrite && __all_sync(0xffffffffu, row_ok)) {
+        uint8_t* slab = sQ + warp * (2 * SLAB_BYTES);
+        uint32_t a[32];
+        tmem_ld_32x32b_x32(tmem_base + lane_base + 256 + col0, a);
+        tmem_wait_ld();
+        store_slab(&tmGV, slab, a, 1.f, p.out_bf16, lane, col0, hk, j * BT + lq * 32, b);
+        tmem_ld_32x32b_x32(tmem_base + lane_base + 384 + col0, a);
+        tmem_wait_ld();
+        store_slab(&tmGK, slab + SLAB_BYTES, a, p.scale, p.out_bf16, lane, col0, hk, j * BT + lq * 32, b);
+        if (lane == 0) tma_store_wait<0>();
+      } else if (row_ok) {
         const size_t row_off = (((size_t)b * p.Skv + (size_t)j * BT + r) * p.Hkv + hk) * HD + col0;
         float* dv_row = p.dv + row_off;
         float* dk_row = p.dk + row_off;
@@ -533,6 +631,16 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       if (!ok && lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/23, (int)n);
     }
+  } else if (n_items == 0 && p.kv_overwrite && warp < KW_COMPUTE) {   // no query sees this tile
+    uint32_t a[32] = {0};
+    uint8_t* slab = sQ + warp * SLAB_BYTES;
+    const int col = (warp >> 2) * 32, row = j * BT + (warp & 3) * 32;
+    store_slab(&tmGV, slab, a, 1.f, p.out_bf16, lane, col, hk, row, b);
+    if (lane == 0) {
+      tma_store_4d(&tmGK, slab, col, hk, row, b);
+      tma_store_commit();
+      tma_store_wait<0>();
+    }
   }
 
   tc_fence_before();
@@ -546,36 +654,43 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // ------------------------------------------------------------------------------------------
 // dQ
 // ------------------------------------------------------------------------------------------
-// K lives until dQ of its item has been issued, V only until dP: a 3-deep K ring and a 2-deep V
-// ring free every slot a full iteration before its next tile is needed (hides the TMA latency).
-constexpr int K_STAGES = 3, V_STAGES = 2;
-constexpr int DQ_SMEM = 2 * TILE_BYTES /*Q,dO*/ + (K_STAGES + V_STAGES) * TILE_BYTES + 1024 + 256;   // barriers: 21 x 8 B
+// K lives until dQ of its item has been issued, V only until dP.
+constexpr int K_STAGES = 4, V_STAGES = 3;
+// Sixteen compute warps like the dK/dV kernel, one TMA warp, two MMA warps.
+constexpr int QW_TMA = 16, QW_MMA = 17, QW_MMA_DQ = 18;
+constexpr int DQ_THREADS = (KW_COMPUTE + 3) * 32;
+constexpr int DQ_ALIGN_SLACK = 768, DQ_BAR_BYTES = 256;   // barriers: 28 x 8 B
+constexpr int DQ_SMEM = (K_STAGES + V_STAGES) * TILE_BYTES + DQ_ALIGN_SLACK + DQ_BAR_BYTES;
+static_assert(DQ_SMEM <= 227 * 1024, "dQ kernel shared memory");
 
 template <bool SPARSE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(DQ_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
-                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdParams p) {
+                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                   const __grid_constant__ CUtensorMap tmGQ, BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sdO = smem + TILE_BYTES;
-  uint8_t* sK = smem + 2 * TILE_BYTES;            // [K_STAGES]
+  uint8_t* sK = smem;                             // [K_STAGES]
   uint8_t* sV = sK + K_STAGES * TILE_BYTES;       // [V_STAGES]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + V_STAGES * TILE_BYTES);
-  uint64_t* qdo_full = bars;       // 1
-  uint64_t* k_full = bars + 1;     // [3]
-  uint64_t* k_empty = bars + 4;    // [3]
-  uint64_t* v_full = bars + 7;     // [2]
-  uint64_t* v_empty = bars + 9;    // [2]
-  uint64_t* s_full = bars + 11;    // 1
-  uint64_t* dp_full = bars + 12;   // 1
-  uint64_t* s_read = bars + 13;    // 1 (one arrival per compute warp)
-  uint64_t* ds_ready = bars + 14;  // 1 (one arrival per compute warp)
-  uint64_t* acc_done = bars + 15;  // 1
-  uint64_t* drain_bar = bars + 16; // [2]
-  uint64_t* dp_free = bars + 18;   // [2] dQ of the item that used this dP buffer has finished reading it
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t* k_full = bars;          // [4]
+  uint64_t* k_empty = bars + 4;     // [4]
+  uint64_t* v_full = bars + 8;      // [3]
+  uint64_t* v_empty = bars + 11;    // [3]
+  uint64_t* s_full = bars + 14;     // [2] S of key half h is in TMEM
+  uint64_t* dp_full = bars + 16;    // [2]
+  uint64_t* s_read = bars + 18;     // [2] (one arrival per compute warp of the half)
+  uint64_t* ds_ready = bars + 20;   // [2]
+  uint64_t* acc_done = bars + 22;   // 1
+  uint64_t* drain_bar = bars + 23;  // [2]
+  uint64_t* ab_ready = bars + 25;   // 1 Q and dO are in TMEM (one arrival per compute warp)
+  uint64_t* qdo_full = bars + 26;   // 1 Q and dO are in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  if (smem - smem_raw > DQ_ALIGN_SLACK) {  // same verdict in every thread
+    if (threadIdx.x == 0) report(p.status, ZX_ERR_ARG, /*site=*/20, (int)(smem - smem_raw));
+    return;
+  }
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -586,7 +701,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int qpos0 = q_tile_pos(p, t);
 
   if (threadIdx.x == 0) {
-    mbar_init(qdo_full, 1);
     for (int s = 0; s < K_STAGES; ++s) {
       mbar_init(&k_full[s], 1);
       mbar_init(&k_empty[s], 1);
@@ -595,19 +709,20 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 1);
     }
-    mbar_init(s_full, 1);
-    mbar_init(dp_full, 1);
-    mbar_init(s_read, N_COMPUTE / 32);    // per-warp arrivals
-    mbar_init(ds_ready, N_COMPUTE / 32);
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&s_full[h], 1);
+      mbar_init(&dp_full[h], 1);
+      mbar_init(&s_read[h], KW_COMPUTE / 2);    // per-warp arrivals
+      mbar_init(&ds_ready[h], KW_COMPUTE / 2);
+      mbar_init(&drain_bar[h], 1);
+    }
     mbar_init(acc_done, 1);
-    mbar_init(&drain_bar[0], 1);
-    mbar_init(&drain_bar[1], 1);
-    mbar_init(&dp_free[0], 1);
-    mbar_init(&dp_free[1], 1);
+    mbar_init(ab_ready, KW_COMPUTE);
+    mbar_init(qdo_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == W_MMA) {
+  if (warp == QW_MMA) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
@@ -615,38 +730,43 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // TMEM columns: S of both key halves | dP of both (dS over it) | dQ | Q | dO
+  constexpr uint32_t C_DP = 128, C_DQ = 256, C_Q = 384, C_DO = 448;
 
-  int n_items = 0;
-  {
-    KvWalk<SPARSE> w;
-    for (w.init(); w.next(p, qpos0);) ++n_items;
-  }
+  const int n_items = KvWalk<SPARSE>::count(p, qpos0);
 
   if (n_items > 0) {
-    if (warp == W_TMA) {
+    if (warp == QW_TMA) {
       if (lane == 0) {
-        tma_prefetch_desc(&tmK);
-        tma_prefetch_desc(&tmV);
+        // Q and dO pass through the last K and V stages on their way to TMEM: those stages are not needed before items
+        // K_STAGES - 1 and V_STAGES - 1, and waited for below. (Reading the rows from global memory straight into
+        // registers, 16 bytes of 32 different rows per load, took 3 us of every block's start.)
+        uint8_t* sQ = sK + (K_STAGES - 1) * TILE_BYTES;
+        uint8_t* sdO = sV + (V_STAGES - 1) * TILE_BYTES;
         mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
         tma_load_4d(sQ, &tmQ, qdo_full, 0, hq, t * BT, b);
         tma_load_4d(sQ + HALF_BYTES, &tmQ, qdo_full, 64, hq, t * BT, b);
         tma_load_4d(sdO, &tmdO, qdo_full, 0, hq, t * BT, b);
         tma_load_4d(sdO + HALF_BYTES, &tmdO, qdo_full, 64, hq, t * BT, b);
         uint32_t n = 0;
+        int ks = 0, vs = 0;
+        uint32_t kph = 1, vph = 1;
         bool ok = true;
         KvWalk<SPARSE> w;
-        for (w.init(); w.next(p, qpos0);) {
+        for (w.init(); w.next(p, qpos0); ++n) {
           const int j = w.j;
-          const int ks = n % K_STAGES, vs = n % V_STAGES;
-          if (!mbar_wait(&k_empty[ks], ((n / K_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(&k_empty[ks], kph, abort_flag)) { ok = false; break; }
+          if (n == K_STAGES - 1 && !mbar_wait(ab_ready, 0, abort_flag)) { ok = false; break; }
           mbar_expect_tx(&k_full[ks], TILE_BYTES);
           tma_load_4d(sK + ks * TILE_BYTES, &tmK, &k_full[ks], 0, hk, j * BT, b);
           tma_load_4d(sK + ks * TILE_BYTES + HALF_BYTES, &tmK, &k_full[ks], 64, hk, j * BT, b);
-          if (!mbar_wait(&v_empty[vs], ((n / V_STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (++ks == K_STAGES) { ks = 0; kph ^= 1u; }
+          if (!mbar_wait(&v_empty[vs], vph, abort_flag)) { ok = false; break; }
+          if (n == V_STAGES - 1 && !mbar_wait(ab_ready, 0, abort_flag)) { ok = false; break; }
           mbar_expect_tx(&v_full[vs], TILE_BYTES);
           tma_load_4d(sV + vs * TILE_BYTES, &tmV, &v_full[vs], 0, hk, j * BT, b);
           tma_load_4d(sV + vs * TILE_BYTES + HALF_BYTES, &tmV, &v_full[vs], 64, hk, j * BT, b);
-          ++n;
+          if (++vs == V_STAGES) { vs = 0; vph ^= 1u; }
         }
         if (!ok) {
           report(p.status, ZX_ERR_TIMEOUT, /*site=*/21, (int)n);
@@ -655,44 +775,24 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           }
         }
       }
-    } else if (warp == W_MMA) {
-      // MMA warp of the "early" products: S(n+1) = Q K(n+1)^T as soon as the compute warps hold S(n) in
-      // registers, dP(n+1) = dO V(n+1)^T into the dP buffer that dQ(n-1) has released. A tcgen05.mma leaves
-      // its issuing thread only when the tensor core has room for it, so these must not queue behind dQ(n)
-      // in one warp's instruction stream: dQ has a warp of its own (below). dP lives in two TMEM buffers
-      // used alternately; with that the compute warps never wait for a tensor result of their own item.
-      constexpr uint32_t idesc_kk = make_idesc(BT, BT, 1, 1, 0, 0);
-      const uint32_t t_s = tmem_base, t_dp = tmem_base + 128;
-      const uint64_t q_addr = base_kmajor(smem_u32(sQ)), do_addr = base_kmajor(smem_u32(sdO));
-      const uint64_t k_k0 = base_kmajor(smem_u32(sK)), v_k0 = base_kmajor(smem_u32(sV));
-      bool ok = mbar_wait_w(qdo_full, 0, abort_flag);
-      ok = ok && mbar_wait_w(&k_full[0], 0, abort_flag);
-      ok = ok && mbar_wait_w(&v_full[0], 0, abort_flag);
-      tc_fence_after();
-      if (ok) {
-        umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_s, q_addr, k_k0, idesc_kk, 0u);
-        umma_commit_w(s_full);
-        umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_dp, do_addr, v_k0, idesc_kk, 0u);
-        umma_commit_w(dp_full);
-        umma_commit_w(&v_empty[0]);
-      }
-      int n = 0;
-      for (; n + 1 < n_items && ok; ++n) {
-        const int ksn = (n + 1) % K_STAGES, vsn = (n + 1) % V_STAGES;
-        const uint64_t kn_addr = desc_advance(k_k0, (uint32_t)ksn * TILE_BYTES);
-        const uint64_t vn_addr = desc_advance(v_k0, (uint32_t)vsn * TILE_BYTES);
-        if (!mbar_wait_w(s_read, n & 1, abort_flag)) { ok = false; break; }
-        if (!mbar_wait_w(&k_full[ksn], ((n + 1) / K_STAGES) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_s, q_addr, kn_addr, idesc_kk, 0u);
-        umma_commit_w(s_full);
-        // buffer (n+1) & 1 held dS(n-1), which dQ(n-1) reads
-        if (n >= 1 && !mbar_wait_w(&dp_free[(n + 1) & 1], ((n - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
-        if (!mbar_wait_w(&v_full[vsn], ((n + 1) / V_STAGES) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        umma_ss_k8_kmajor_w<HALF_BYTES / 16>(t_dp + (uint32_t)((n + 1) & 1) * 256, do_addr, vn_addr, idesc_kk, 0u);
-        umma_commit_w(dp_full);
-        umma_commit_w(&v_empty[vsn]);   // V(n+1) is only read by dP(n+1)
+    } else if (warp == QW_MMA) {
+      // S_h(n+1) = Q K_h(n+1)^T as soon as the half's warps hold S_h(n) in registers
+      constexpr uint32_t idesc_kk = make_idesc(BT, BT / 2, 1, 1, 0, 0);
+      const uint64_t k_k0 = base_kmajor(smem_u32(sK));
+      bool ok = mbar_wait_w(ab_ready, 0, abort_flag);
+      int n = 0, ks = 0;
+      uint32_t kph = 0;
+      for (; n < n_items && ok; ++n) {
+        for (int h = 0; h < 2; ++h) {
+          const bool got = h == 0 ? mbar_wait2_w(&s_read[0], (n & 1) ^ 1, &k_full[ks], kph, abort_flag)
+                                  : mbar_wait_w(&s_read[1], (n & 1) ^ 1, abort_flag);
+          if (!got) { ok = false; break; }
+          tc_fence_after();
+          umma_ts_k8_kmajor_w<HALF_BYTES / 16>(tmem_base + 64 * h, tmem_base + C_Q,
+                                               desc_advance(k_k0, (uint32_t)ks * TILE_BYTES + h * HALF_Q), idesc_kk, 0u);
+          umma_commit_w(&s_full[h]);
+        }
+        if (++ks == K_STAGES) { ks = 0; kph ^= 1u; }
       }
       if (!ok) {
         if (lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/22, n);
@@ -701,23 +801,39 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         while (!mbar_try_wait(&drain_bar[0], 0) && globaltimer_ns() - t0 < 50000000ull) {
         }
       }
-    } else if (warp == W_MMA_DQ) {
-      // MMA warp of dQ(n) += dS(n) K(n): A = dS from the dP buffer of item n, B = K(n) read transposed
+    } else if (warp == QW_MMA_DQ) {
+      // dQ += dS_h(n) K_h(n) (dS from TMEM, K read transposed), then dP_h(n+1) = dO V_h(n+1)^T over that dS
+      constexpr uint32_t idesc_kk = make_idesc(BT, BT / 2, 1, 1, 0, 0);
       constexpr uint32_t idesc_tm = make_idesc(BT, HD, 1, 1, 0, 1);
-      const uint32_t t_dp = tmem_base + 128, t_dq = tmem_base + 256;
-      const uint64_t k_mn0 = base_mnmajor(smem_u32(sK));
-      bool ok = true;
-      int n = 0;
+      const uint64_t k_mn0 = base_mnmajor(smem_u32(sK)), v_k0 = base_kmajor(smem_u32(sV));
+      auto dprob = [&](int h, int vs) {
+        umma_ts_k8_kmajor_w<HALF_BYTES / 16>(tmem_base + C_DP + 64 * h, tmem_base + C_DO,
+                                             desc_advance(v_k0, (uint32_t)vs * TILE_BYTES + h * HALF_Q), idesc_kk, 0u);
+        umma_commit_w(&dp_full[h]);
+      };
+      bool ok = mbar_wait_w(ab_ready, 0, abort_flag);
+      ok = ok && mbar_wait_w(&v_full[0], 0, abort_flag);
+      tc_fence_after();
+      if (ok) {
+        dprob(0, 0);
+        dprob(1, 0);
+      }
+      int n = 0, ks = 0, vs = 1;   // V stage of item n + 1
+      uint32_t vph = 0;
       for (; n < n_items && ok; ++n) {
-        const int ks = n % K_STAGES;
-        if (!mbar_wait_w(ds_ready, n & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        if (lane == 0) ZX_TRACE(n, 8);
-        umma_ts_k8_w<8, 16, 24, 64, 72, 80, 88>(t_dq, t_dp + (uint32_t)(n & 1) * 256,
-                                                 desc_advance(k_mn0, (uint32_t)ks * TILE_BYTES), idesc_tm, n > 0 ? 1u : 0u);
-        umma_commit_w(&k_empty[ks]);        // K(n) has now served S(n) and dQ(n)
-        umma_commit_w(&dp_free[n & 1]);
-        if (lane == 0) ZX_TRACE(n, 9);
+        const bool has_next = n + 1 < n_items;
+        for (int h = 0; h < 2; ++h) {
+          const bool got = h == 0 && has_next ? mbar_wait2_w(&ds_ready[0], n & 1, &v_full[vs], vph, abort_flag)
+                                              : mbar_wait_w(&ds_ready[h], n & 1, abort_flag);
+          if (!got) { ok = false; break; }
+          tc_fence_after();
+          umma_ts_k4_w<8, 32, 40>(tmem_base + C_DQ, tmem_base + C_DP + 64 * h,
+                                  desc_advance(k_mn0, (uint32_t)ks * TILE_BYTES + h * HALF_Q), idesc_tm, (n > 0 || h > 0) ? 1u : 0u);
+          if (has_next) dprob(h, vs);
+        }
+        if (!ok) break;
+        if (++ks == K_STAGES) ks = 0;
+        if (++vs == V_STAGES) { vs = 0; vph ^= 1u; }
       }
       if (ok) umma_commit_w(acc_done);
       if (!ok) {
@@ -728,108 +844,123 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
     } else {
-      // Two warpgroups: warpgroup wg owns key columns [64 wg, 64 wg + 64) of every query row.
+      // Column group wg owns key columns [32 wg, 32 wg + 32) of every query row; groups 0, 1 are key half 0, 2, 3 half 1.
       const int wg = warp >> 2;
+      const int half = wg >> 1;
       const int lq = warp & 3;
       const int r = lq * 32 + lane;  // query row == TMEM lane
-      const int col0 = wg * 64;
+      const int col0 = wg * 32;
       const uint32_t lane_base = (uint32_t)(lq * 32) << 16;
-      const uint32_t t_s = tmem_base + lane_base + col0, t_dp0 = tmem_base + lane_base + 128 + col0;
-      const size_t stat_idx = ((size_t)b * p.Hq + hq) * p.Sq + (size_t)t * BT + r;
-      const float lse2 = p.lse[stat_idx] * LOG2E;
-      const float dlt = p.delta[stat_idx];
-      const int my_qpos = qpos0 + r;
-      uint32_t n = 0;
       bool ok = true;
-      KvWalk<SPARSE> walk;
-      for (walk.init(); walk.next(p, qpos0);) {
-        const int kpos0 = walk.kpos0;
-        if (!wait_warp(s_full, n & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        if (threadIdx.x == 0) ZX_TRACE(n, 0);
-        if (threadIdx.x == 160) ZX_TRACE(n, 11);
-        uint32_t sr[64];
-        tmem_ld_32x32b_x32(t_s + 0, sr);
-        tmem_ld_32x32b_x32(t_s + 32, sr + 32);
-        tmem_wait_ld();
-        if (threadIdx.x == 0) ZX_TRACE(n, 1);
+      const uint32_t t_s = tmem_base + lane_base + col0, t_dp = t_s + C_DP;
+      {
+        // Q and dO of this tile into TMEM, where they are the A operands of S and dP (as shared-memory operands they
+        // would make 128 x 64 products wait for shared memory: 6 KB per 32 clk of MMA). Groups 0 and 1 take the two
+        // halves of the head dimension of Q, 2 and 3 of dO: 64 values of one row per thread, two per 32-bit column.
+        const uint8_t* src = (wg < 2 ? sK + (K_STAGES - 1) * TILE_BYTES : sV + (V_STAGES - 1) * TILE_BYTES) +
+                             (wg & 1) * HALF_BYTES + r * 128;
+        if (!mbar_wait_w(qdo_full, 0, abort_flag)) ok = false;
+        uint32_t x[32];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 u = *reinterpret_cast<const uint4*>(src + ((i ^ (r & 7)) << 4));   // 128-byte swizzle
+          x[4 * i] = u.x; x[4 * i + 1] = u.y; x[4 * i + 2] = u.z; x[4 * i + 3] = u.w;
+        }
+        tmem_st_32x32b_x32(tmem_base + lane_base + C_Q + col0, x);
+        tmem_wait_st();
+        fence_proxy_async_smem();   // the stages are refilled by TMA once every warp has arrived
         tc_fence_before();
-        mbar_arrive_warp(s_read);
-        const bool diag = p.causal && (kpos0 + BT - 1 > qpos0);
-        const int kp = kpos0 + col0;
+        mbar_arrive_warp(ab_ready);
+      }
+      const size_t stat_idx = ((size_t)b * p.Hq + hq) * p.Sq + (size_t)t * BT + r;
+      const float nlse2 = -p.lse[stat_idx] * LOG2E;
+      const float ndlt = -p.delta[stat_idx];
+      uint32_t n = 0;
+      int vs = 0;
+      KvWalk<SPARSE> walk;
+      for (walk.init(); ok && walk.next(p, qpos0); ++n) {
+        if (!wait_warp(&s_full[half], n & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t sr[32];
+        tmem_ld_32x32b_x32(t_s, sr);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive_warp(&s_read[half]);
         const float2 sl2 = make_float2(p.scale_log2, p.scale_log2);
-        const float2 nl2 = make_float2(-lse2, -lse2);
-        static_for<32>([&](auto idx) {   // packed fp32x2 math: two key columns per instruction
+        const float2 nl2 = make_float2(nlse2, nlse2);
+        static_for<16>([&](auto idx) {   // packed fp32x2 math: two key columns per instruction
           constexpr int c = decltype(idx)::value;
           const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[2 * c]), __uint_as_float(sr[2 * c + 1])), sl2, nl2);
           const float2 e = exp2_pair<c, DQ_POLY_EVERY>(x);
           sr[2 * c] = __float_as_uint(e.x);
           sr[2 * c + 1] = __float_as_uint(e.y);
         });
-        if (diag) {   // only tiles on the diagonal pay for the per-element mask
+        if (p.causal && walk.kpos0 + BT - 1 > qpos0) {   // only tiles on the diagonal pay for the per-element mask
+          const int last = qpos0 + r - walk.kpos0 - col0;   // columns up to this one are visible to the row
 #pragma unroll
-          for (int c = 0; c < 64; ++c)
-            if (kp + c > my_qpos) sr[c] = 0u;
+          for (int c = 0; c < 32; ++c)
+            if (c > last) sr[c] = 0u;
         }
-        if (threadIdx.x == 0) ZX_TRACE(n, 2);
-        if (threadIdx.x == 160) ZX_TRACE(n, 12);
-        if (!wait_warp(dp_full, n & 1, abort_flag)) { ok = false; break; }
+        if (!wait_warp(&dp_full[half], n & 1, abort_flag)) { ok = false; break; }
+        // dP of half 1 was issued after dQ(n-1): its arrival says that K(n-1) and V(n) have been read. Handed back here
+        // and not by commits of the issuing warp, whose queue they would fill.
+        if (threadIdx.x == 256) {
+          if (n > 0) mbar_arrive(&k_empty[(n - 1) % K_STAGES]);
+          mbar_arrive(&v_empty[vs]);
+          vs = vs + 1 == V_STAGES ? 0 : vs + 1;
+        }
         tc_fence_after();
-        if (threadIdx.x == 0) ZX_TRACE(n, 3);
-        const uint32_t t_dp = t_dp0 + (n & 1) * 256;   // the two dP buffers sit at columns 128 and 384
-        uint32_t dp[64];
-        tmem_ld_32x32b_x32(t_dp + 0, dp);
-        tmem_ld_32x32b_x32(t_dp + 32, dp + 32);
+        uint32_t dp[32];
+        tmem_ld_32x32b_x32(t_dp, dp);
         tmem_wait_ld();
-        if (threadIdx.x == 0) ZX_TRACE(n, 4);
         {
-          uint32_t dsp[32];
-          const float2 ndl = make_float2(-dlt, -dlt);
+          uint32_t dsp[16];
+          const float2 ndl = make_float2(ndlt, ndlt);
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
+          for (int e = 0; e < 16; ++e) {
             const float2 t2 = __fadd2_rn(make_float2(__uint_as_float(dp[2 * e]), __uint_as_float(dp[2 * e + 1])), ndl);
             const float2 d = __fmul2_rn(make_float2(__uint_as_float(sr[2 * e]), __uint_as_float(sr[2 * e + 1])), t2);
             dsp[e] = pack_bf16x2(d.x, d.y);
           }
-          if (threadIdx.x == 0) ZX_TRACE(n, 6);
-          tmem_st_32x32b_x32(t_dp, dsp);   // bf16 dS for this half, over the columns this thread just read
+          tmem_st_32x32b_x16(t_dp, dsp);   // bf16 dS over the first 16 of the 32 columns this thread just read
         }
         tmem_wait_st();
-        if (threadIdx.x == 0) ZX_TRACE(n, 5);
-        if (threadIdx.x == 160) ZX_TRACE(n, 13);
         tc_fence_before();
-        mbar_arrive_warp(ds_ready);
-        ++n;
+        mbar_arrive_warp(&ds_ready[half]);
       }
       if (ok) ok = wait_warp(acc_done, 0, abort_flag);
       tc_fence_after();
-      if (ok && ZX_IN_BOUNDS(p.status, t * BT + r, p.Sq, 25)) {
+      const bool row_ok = ok && ZX_IN_BOUNDS(p.status, t * BT + r, p.Sq, 25);
+      if (!p.dq_accumulate && __all_sync(0xffffffffu, row_ok)) {
+        uint32_t a[32];
+        tmem_ld_32x32b_x32(tmem_base + lane_base + C_DQ + col0, a);
+        tmem_wait_ld();
+        store_slab(&tmGQ, sK + warp * SLAB_BYTES, a, p.scale, p.out_bf16, lane, col0, hq, t * BT + lq * 32, b);
+        if (lane == 0) tma_store_wait<0>();
+      } else if (row_ok) {
         float* dq_row = p.dq + (((size_t)b * p.Sq + (size_t)t * BT + r) * p.Hq + hq) * HD + col0;
+        uint32_t a[32];
+        tmem_ld_32x32b_x32(tmem_base + lane_base + C_DQ + col0, a);
+        tmem_wait_ld();
+        float4* dst = reinterpret_cast<float4*>(dq_row);
 #pragma unroll
-        for (int ci = 0; ci < 2; ++ci) {
-          uint32_t a[32];
-          tmem_ld_32x32b_x32(tmem_base + lane_base + 256 + col0 + ci * 32, a);
-          tmem_wait_ld();
-          float4* dst = reinterpret_cast<float4*>(dq_row + ci * 32);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            float4 v = make_float4(__uint_as_float(a[4 * e]) * p.scale, __uint_as_float(a[4 * e + 1]) * p.scale,
-                                   __uint_as_float(a[4 * e + 2]) * p.scale, __uint_as_float(a[4 * e + 3]) * p.scale);
-            if (p.dq_accumulate) {
-              const float4 o = dst[e];
-              v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-            }
-            dst[e] = v;
-          }
+        for (int e = 0; e < 8; ++e) {
+          const float4 o = dst[e];
+          dst[e] = make_float4(o.x + __uint_as_float(a[4 * e]) * p.scale, o.y + __uint_as_float(a[4 * e + 1]) * p.scale,
+                               o.z + __uint_as_float(a[4 * e + 2]) * p.scale, o.w + __uint_as_float(a[4 * e + 3]) * p.scale);
         }
       }
       if (!ok && lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/23, (int)n);
     }
+  } else if (n_items == 0 && !p.dq_accumulate && warp < KW_COMPUTE) {   // this tile sees no key
+    uint32_t a[32] = {0};
+    store_slab(&tmGQ, sK + warp * SLAB_BYTES, a, 1.f, p.out_bf16, lane, (warp >> 2) * 32, hq, t * BT + (warp & 3) * 32, b);
+    if (lane == 0) tma_store_wait<0>();
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == W_MMA) {
+  if (warp == QW_MMA) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
@@ -840,6 +971,15 @@ CUtensorMap make_qkv_map(const void* base, int B, int S, int H, int64_t tok_stri
   uint64_t strides[3] = {(uint64_t)HD * 2, (uint64_t)tok_stride * 2, (uint64_t)S * (uint64_t)tok_stride * 2};
   uint32_t box[4] = {64, 1, 128, 1};
   return make_tma_map(base, 2, 4, dims, strides, box, TmaSwizzle::B128);
+}
+
+// A gradient [B, S, H, 128], stored 32 columns x 32 rows at a time (one warp's part of an accumulator).
+CUtensorMap make_grad_map(const void* base, int B, int S, int H, int bf16) {
+  const uint64_t es = bf16 ? 2 : 4;
+  uint64_t dims[4] = {(uint64_t)HD, (uint64_t)H, (uint64_t)S, (uint64_t)B};
+  uint64_t strides[3] = {HD * es, (uint64_t)H * HD * es, (uint64_t)S * (uint64_t)H * HD * es};
+  uint32_t box[4] = {32, 1, 32, 1};
+  return make_tma_map(base, (int)es, 4, dims, strides, box, bf16 ? TmaSwizzle::B64 : TmaSwizzle::B128);
 }
 
 template <typename K>
@@ -855,10 +995,9 @@ void launch_attn_bwd(const AttnBwdArgs& a) {
   check_attn_common(a.Hq, a.Hkv, a.Sq, a.Skv, a.q_layout, a.kv_layout);
   if (a.Sq == 0 || a.Skv == 0 || a.B == 0) return;
   if (a.compute_delta) {
-    const size_t rows = (size_t)a.B * a.Sq * a.Hq;
-    const int wpb = 8;
-    attn_delta_kernel<<<(unsigned)((rows + wpb - 1) / wpb), wpb * 32, 0, a.stream>>>(
-        (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.delta, a.B, a.Sq, a.Hq);
+    const int groups = (int)((size_t)a.B * a.Sq * a.Hq / DELTA_TOKENS);
+    attn_delta_kernel<<<(groups + 7) / 8, 256, 0, a.stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.delta,
+                                                              a.Sq, a.Hq, groups);
   }
   CUtensorMap tmQ = make_qkv_map(a.q, a.B, a.Sq, a.Hq, a.q_tok_stride);
   CUtensorMap tmdO = make_qkv_map(a.d_o, a.B, a.Sq, a.Hq, (int64_t)a.Hq * HD);
@@ -873,13 +1012,20 @@ void launch_attn_bwd(const AttnBwdArgs& a) {
   p.n_kv_tiles = a.Skv / BT;
   p.q_tiles_per_chunk = a.q_layout.chunk_len / BT;
   p.kv_tiles_per_chunk = a.kv_layout.chunk_len / BT;
+  p.n_q_chunks = a.q_layout.n_chunks;
+  p.n_kv_chunks = a.kv_layout.n_chunks;
   for (int c = 0; c < kAttnMaxChunks; ++c) {
     p.q_chunk_pos[c] = c < a.q_layout.n_chunks ? a.q_layout.chunk_pos[c] : 0;
     p.kv_chunk_pos[c] = c < a.kv_layout.n_chunks ? a.kv_layout.chunk_pos[c] : 0;
   }
   p.lse = a.lse; p.delta = a.delta;
-  p.dq = a.dq; p.dk = a.dk; p.dv = a.dv;
-  p.dq_accumulate = a.dq_accumulate;
+  if (a.out_bf16 && (a.dq_accumulate || !a.kv_overwrite))
+    throw std::runtime_error("attn_bwd: bf16 gradients can only be written, not added to");
+  p.dq = (float*)a.dq; p.dk = (float*)a.dk; p.dv = (float*)a.dv;
+  p.dq_accumulate = a.dq_accumulate; p.kv_overwrite = a.kv_overwrite; p.out_bf16 = a.out_bf16;
+  const CUtensorMap tmGQ = make_grad_map(a.dq, a.B, a.Sq, a.Hq, a.out_bf16);
+  const CUtensorMap tmGK = make_grad_map(a.dk, a.B, a.Skv, a.Hkv, a.out_bf16);
+  const CUtensorMap tmGV = make_grad_map(a.dv, a.B, a.Skv, a.Hkv, a.out_bf16);
   if (a.pull_bytes % 16 != 0) throw std::runtime_error("attn_bwd: pull size must be a multiple of 16 bytes");
   p.pull_src = (const uint4*)a.pull_src;
   p.pull_dst = (uint4*)a.pull_dst;
@@ -900,11 +1046,11 @@ void launch_attn_bwd(const AttnBwdArgs& a) {
   p.q_heads_per_group = heads_per_group(p.n_kv_tiles, a.B * a.Hq, uniform, false);
   const unsigned grid_kv = p.n_kv_tiles * a.B * a.Hkv, grid_q = p.n_q_tiles * a.B * a.Hq;
   if (p.window_blocks > 0) {
-    attn_bwd_dkdv_kernel<true><<<grid_kv, DKDV_THREADS, DKDV_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, p);
-    attn_bwd_dq_kernel<true><<<grid_q, NUM_THREADS, DQ_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, p);
+    attn_bwd_dkdv_kernel<true><<<grid_kv, DKDV_THREADS, DKDV_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, tmGK, tmGV, p);
+    attn_bwd_dq_kernel<true><<<grid_q, DQ_THREADS, DQ_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, tmGQ, p);
   } else {
-    attn_bwd_dkdv_kernel<false><<<grid_kv, DKDV_THREADS, DKDV_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, p);
-    attn_bwd_dq_kernel<false><<<grid_q, NUM_THREADS, DQ_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, p);
+    attn_bwd_dkdv_kernel<false><<<grid_kv, DKDV_THREADS, DKDV_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, tmGK, tmGV, p);
+    attn_bwd_dq_kernel<false><<<grid_q, DQ_THREADS, DQ_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, tmGQ, p);
   }
 }
 

@@ -177,7 +177,7 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
               Tensor& delta, Tensor& dq, Tensor& dk, Tensor& dv, double scale, bool causal, int64_t window_blocks,
               int64_t global_every, const std::vector<int64_t>& q_chunk_pos, const std::vector<int64_t>& kv_chunk_pos,
               bool compute_delta, bool dq_accumulate, int64_t pull_src, int64_t pull_dst, int64_t pull_bytes,
-              const c10::optional<Tensor>& trace) {
+              const c10::optional<Tensor>& trace, bool kv_overwrite) {
   check_qkv(q, "q");
   check_qkv(k, "k");
   check_qkv(v, "v");
@@ -185,7 +185,11 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
   check_bf16(d_o, "d_o");
   TORCH_CHECK(o.is_contiguous() && d_o.is_contiguous() && o.sizes() == q.sizes() && d_o.sizes() == q.sizes(),
               "o and d_o must be contiguous with q's shape");
-  for (const Tensor* t : std::initializer_list<const Tensor*>{&lse, &delta, &dq, &dk, &dv})
+  const bool out_bf16 = dq.scalar_type() == torch::kBFloat16;
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&dq, &dk, &dv})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == dq.scalar_type() && t->is_contiguous() &&
+                    (out_bf16 || t->scalar_type() == torch::kFloat32), "gradients: contiguous, all fp32 or all bf16");
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&lse, &delta})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->is_contiguous(), "fp32 contiguous expected");
   TORCH_CHECK(dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == v.sizes(), "gradient shapes differ");
   TORCH_CHECK(delta.sizes() == lse.sizes(), "delta must match lse");
@@ -193,7 +197,8 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
   zx::AttnBwdArgs a;
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.d_o = d_o.data_ptr();
   a.lse = lse.data_ptr<float>(); a.delta = delta.data_ptr<float>();
-  a.dq = dq.data_ptr<float>(); a.dk = dk.data_ptr<float>(); a.dv = dv.data_ptr<float>();
+  a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr();
+  a.out_bf16 = out_bf16; a.kv_overwrite = kv_overwrite;
   a.B = (int)q.size(0); a.Sq = (int)q.size(1); a.Hq = (int)q.size(2);
   a.Skv = (int)k.size(1); a.Hkv = (int)k.size(2);
   a.q_tok_stride = q.stride(1); a.k_tok_stride = k.stride(1); a.v_tok_stride = v.stride(1);
@@ -514,7 +519,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("delta"), py::arg("dq"), py::arg("dk"), py::arg("dv"), py::arg("scale"), py::arg("causal"),
         py::arg("window_blocks"), py::arg("global_every"), py::arg("q_chunk_pos"), py::arg("kv_chunk_pos"),
         py::arg("compute_delta"), py::arg("dq_accumulate"), py::arg("pull_src"), py::arg("pull_dst"),
-        py::arg("pull_bytes"), py::arg("trace") = py::none());
+        py::arg("pull_bytes"), py::arg("trace") = py::none(), py::arg("kv_overwrite") = false);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("rope_qkv", &rope_qkv);

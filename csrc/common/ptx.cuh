@@ -128,6 +128,12 @@ __device__ __forceinline__ bool mbar_wait_w(uint64_t* bar, uint32_t parity, vola
   const bool ok = mbar_wait(bar, parity, abort_flag);
   return __all_sync(0xffffffffu, ok);
 }
+// Both barriers at once: two waits one after the other cost an issuing warp twice the latency of the poll.
+__device__ __forceinline__ bool mbar_wait2_w(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, volatile int* abort_flag) {
+  const bool ra = mbar_try_wait(a, pa), rb = mbar_try_wait(b, pb);
+  if (__all_sync(0xffffffffu, ra && rb)) return true;
+  return mbar_wait_w(a, pa, abort_flag) && mbar_wait_w(b, pb, abort_flag);
+}
 
 // ----------------------------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies). Every load targets the issuing CTA only.
@@ -160,6 +166,12 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(m)),
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* smem_src, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }

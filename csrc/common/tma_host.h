@@ -25,7 +25,7 @@ inline PFN_encodeTiled get_encode_tiled() {
   return fn;
 }
 
-enum class TmaSwizzle { None, B128 };
+enum class TmaSwizzle { None, B64, B128 };
 
 // Generic tiled map, up to rank 4. dims[0] is the contiguous dimension. strides_bytes[i] is the
 // byte stride of dims[i+1] (rank-1 entries), each a multiple of 16. box[0]*elem_size must be
@@ -51,7 +51,9 @@ inline CUtensorMap make_tma_map(const void* base, int elem_bytes, int rank, cons
                                              : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   CUresult r = get_encode_tiled()(&m, dt, (cuuint32_t)rank, const_cast<void*>(base), gdims, gstr, bx, es,
                                   CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                  swz == TmaSwizzle::B128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                                  swz == TmaSwizzle::B128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                  : swz == TmaSwizzle::B64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                           : CU_TENSOR_MAP_SWIZZLE_NONE,
                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
   return m;

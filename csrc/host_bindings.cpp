@@ -7,6 +7,7 @@
 #include "cpu_ref/flash_cpu.h"
 #include "cpu_ref/quant_adamw_ref.h"
 #include "attn/tile_iter_host.h"
+#include "attn/work_order.h"
 #include "peer/barrier_model.h"
 #include "tier/belady_min.h"
 #include "tier/tier_engine.h"
@@ -71,6 +72,15 @@ PYBIND11_MODULE(_host, m) {
                                decay_end, lr, beta1, beta2, eps, weight_decay, step);
   }, "in place on p_hi (bf16 bits), p_lo, m, v");
 
+  m.def("attn_work_order", [](int n_tiles, int n_heads, int longest, bool uniform, bool all) {
+    const int per = zx::heads_per_group(longest, n_heads, uniform, all);
+    std::vector<std::pair<int, int>> order;
+    for (int b = 0; b < n_tiles * n_heads; ++b) {
+      const zx::WorkItem w = zx::work_item(b, n_tiles, n_heads, per);
+      order.emplace_back(w.tile, w.head);
+    }
+    return std::make_pair(per, order);
+  }, py::arg("n_tiles"), py::arg("n_heads"), py::arg("longest"), py::arg("uniform"), py::arg("all"));
   m.def("tile_iter_mismatches", &zx::tile_iter_mismatches, py::arg("causal"), py::arg("window_blocks"),
         py::arg("global_every"), py::arg("q_chunk_pos"), py::arg("kv_chunk_pos"), py::arg("q_tiles_per_chunk"),
         py::arg("kv_tiles_per_chunk"));

@@ -1,0 +1,57 @@
+"""Block order of the attention launches (csrc/attn/work_order.h) on the CPU, and the backward kernels at the edges of
+their tiles, item counts and output forms on a GPU."""
+import math
+
+import pytest
+import torch
+
+from zenyx_b200.ops import _ext
+from zenyx_b200.ops.attention import MaskSpec, attn_backward, attn_forward
+
+
+@pytest.mark.parametrize("n_tiles", [1, 2, 3, 17, 64, 256, 300])
+@pytest.mark.parametrize("n_heads", [1, 3, 8, 32])
+@pytest.mark.parametrize("uniform,everything", [(False, False), (True, False), (False, True)])
+def test_block_order_takes_every_tile_of_every_head_once(n_tiles, n_heads, uniform, everything):
+    per, order = _ext.host().attn_work_order(n_tiles, n_heads, n_tiles, uniform, everything)
+    assert 1 <= per <= n_heads
+    assert sorted(order) == [(t, h) for t in range(n_tiles) for h in range(n_heads)]
+    groups = [order[i: i + n_tiles * per] for i in range(0, len(order), n_tiles * per)]
+    for g, blocks in enumerate(groups):
+        assert [t for t, _ in blocks] == sorted(t for t, _ in blocks)             # longest first inside a group
+        assert {h for _, h in blocks} == set(range(g * per, min(n_heads, (g + 1) * per)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,causal,wb,ge,qpos,kpos", [
+    (1, 128, 128, 1, 1, True, 0, 0, [0], [0]),                  # one item, one block
+    (2, 128, 256, 2, 1, False, 0, 0, [0], [0]),                 # two items per block: every stage used once
+    (1, 640, 640, 3, 3, True, 0, 0, [0], [0]),                  # 1 to 5 items: all stage counts wrap
+    (1, 512, 768, 4, 2, True, 0, 0, [0, 1024], [256, 896, 512]),   # unsorted chunks; tiles that see and are seen by nothing
+    (1, 1024, 1024, 2, 1, True, 2, 3, [0], [0]),                # window and global tiles
+])
+def test_attention_backward_writes_every_tile(B, Sq, Skv, Hq, Hkv, causal, wb, ge, qpos, kpos, bf16):
+    """The written (not accumulated) gradients, fp32 and bf16, against the fp32 host path. The buffers start as NaN: a
+    tile without work has to be written too. Bound: P and dS are rounded to bf16 (2^-9 each) before products whose
+    terms partly cancel; the accumulating form of the same kernels is held to 2e-2 in test_gpu_kernels.py."""
+    torch.manual_seed(Sq + Skv)
+    mask, scale = MaskSpec(causal, wb, ge), 1.0 / math.sqrt(128)
+    q, do = (torch.randn(B, Sq, Hq, 128).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Skv, Hkv, 128).bfloat16() for _ in range(2))
+    results = []
+    for dev in ("cpu", "cuda"):
+        a = [t.to(dev) for t in (q, k, v, do)]
+        o, lse = torch.empty_like(a[0]), torch.empty(B, Hq, Sq, device=dev)
+        attn_forward(a[0], a[1], a[2], o, lse, scale, mask, qpos, kpos)
+        grads = [torch.full(t.shape, math.nan, device=dev, dtype=torch.bfloat16 if bf16 and dev == "cuda" else torch.float32)
+                 for t in (q, k, v)]
+        attn_backward(*a[:3], o, a[3], lse, torch.empty_like(lse), *grads, scale, mask, qpos, kpos, kv_overwrite=True)
+        results.append([g.float().cpu() for g in grads])
+    _ext.check_status()
+    for ref, got in zip(*results):
+        assert torch.isfinite(got).all()
+        assert (got - ref).norm() <= 2e-2 * ref.norm()
+        # Zero rows: nothing seen, or (window case, row 0) one key, where dP - delta is the difference of two 32-bit sums
+        # of 128 products of unit normals, each off by at most 128 * 2^-24 * sum|terms| ~ 1e-3 * 2^-7 ~ 1e-5.
+        assert got[ref.abs().amax(-1) == 0].abs().amax().item() <= 1e-5 if (ref.abs().amax(-1) == 0).any() else True

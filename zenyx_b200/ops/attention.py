@@ -189,14 +189,16 @@ def attn_forward(q, k, v, o, lse, scale: float, mask: MaskSpec, q_chunk_pos: Seq
 
 def attn_backward(q, k, v, o, d_o, lse, delta, dq, dk, dv, scale: float, mask: MaskSpec,
                   q_chunk_pos: Sequence[int], kv_chunk_pos: Sequence[int], compute_delta: bool = True,
-                  dq_accumulate: bool = False, pull: Optional[Tuple[int, int, int]] = None) -> None:
-    """dq (fp32) is written or accumulated; dk/dv (fp32) are always added to (zero them first).
+                  dq_accumulate: bool = False, pull: Optional[Tuple[int, int, int]] = None,
+                  kv_overwrite: bool = False) -> None:
+    """dq (fp32) is written or accumulated; dk/dv (fp32) are added to (zero them first), or written with
+    ``kv_overwrite``, in which case the three may also be bf16 (each element rounded once, from fp32).
     `lse` must be the final log-sum-exp over *all* keys the queries saw (all ring steps)."""
     if _ext.use_cuda_kernels(q):
         ps, pd, pb = pull if pull is not None else (0, 0, 0)
         _ext.C().attn_bwd(q, k, v, o, d_o, lse, delta, dq, dk, dv, scale, mask.causal, mask.window_blocks,
                           mask.global_every, list(q_chunk_pos), list(kv_chunk_pos), compute_delta, dq_accumulate,
-                          ps, pd, pb)
+                          ps, pd, pb, None, kv_overwrite)
         return
     Hq, Hkv = q.shape[2], k.shape[2]
     G = Hq // Hkv
@@ -220,8 +222,12 @@ def attn_backward(q, k, v, o, d_o, lse, delta, dq, dk, dv, scale: float, mask: M
         dq.add_(dq_cur)
     else:
         dq.copy_(dq_cur)
-    dk.add_(dk_cur)
-    dv.add_(dv_cur)
+    if kv_overwrite:
+        dk.copy_(dk_cur)
+        dv.copy_(dv_cur)
+    else:
+        dk.add_(dk_cur)
+        dv.add_(dv_cur)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -243,12 +249,11 @@ class _FlashAttnFn(torch.autograd.Function):
     def backward(ctx, d_o):
         q, k, v, o, lse = ctx.saved_tensors
         scale, mask, qp, kp = ctx.cfg
-        dq = torch.empty(q.shape, device=q.device, dtype=torch.float32)
-        dk = torch.zeros(k.shape, device=q.device, dtype=torch.float32)
-        dv = torch.zeros(v.shape, device=q.device, dtype=torch.float32)
+        # every gradient tile is produced by one block, so it is rounded to the inputs' type where it is stored
+        dq, dk, dv = (torch.empty(t.shape, device=t.device, dtype=t.dtype) for t in (q, k, v))
         delta = torch.empty_like(lse)
-        attn_backward(q, k, v, o, d_o.contiguous(), lse, delta, dq, dk, dv, scale, mask, qp, kp)
-        return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), None, None, None, None
+        attn_backward(q, k, v, o, d_o.contiguous(), lse, delta, dq, dk, dv, scale, mask, qp, kp, kv_overwrite=True)
+        return dq, dk, dv, None, None, None, None
 
 
 def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = True,
@@ -350,17 +355,19 @@ def ring_attn_forward(ctx: RingContext, q, k, v, scale: float, slot: int = 0):
     return o, lse
 
 
-def ring_attn_backward(ctx: RingContext, q, k, v, o, d_o, lse, scale: float, slot: int = 0):
+def ring_attn_backward(ctx: RingContext, q, k, v, o, d_o, lse, scale: float, slot: int = 0,
+                       grad_dtype: torch.dtype = torch.float32):
     """Backward over all ring steps. Returns (dq fp32, dk fp32, dv fp32) for this rank's tokens;
-    on GPU dk/dv are views of this rank's peer-visible accumulators (valid until the slot is reused)."""
+    on GPU dk/dv are views of this rank's peer-visible accumulators (valid until the slot is reused).
+    ``grad_dtype`` is what a ring of one rank, which adds nothing up, returns them in."""
     B, Sq, Hq, D = q.shape
-    dq = torch.empty(B, Sq, Hq, D, device=q.device, dtype=torch.float32)
     delta = torch.empty_like(lse)
     if ctx.degree == 1:
-        dk = torch.zeros(k.shape, device=q.device, dtype=torch.float32)
-        dv = torch.zeros(v.shape, device=q.device, dtype=torch.float32)
-        attn_backward(q, k, v, o, d_o, lse, delta, dq, dk, dv, scale, ctx.mask, ctx.positions(), ctx.positions())
+        dq, dk, dv = (torch.empty(t.shape, device=t.device, dtype=grad_dtype) for t in (q, k, v))
+        attn_backward(q, k, v, o, d_o, lse, delta, dq, dk, dv, scale, ctx.mask, ctx.positions(), ctx.positions(),
+                      kv_overwrite=True)
         return dq, dk, dv
+    dq = torch.empty(B, Sq, Hq, D, device=q.device, dtype=torch.float32)
     steps = ctx.active_steps(Sq, k.shape[1])
     if not q.is_cuda:
         import torch.distributed as dist
@@ -431,7 +438,7 @@ class _RingAttnFn(torch.autograd.Function):
             ks.copy_(k)
             vs.copy_(v)
             k, v = ks, vs
-        dq, dk, dv = ring_attn_backward(ring, q, k, v, o, d_o.contiguous(), lse, scale, 0)
+        dq, dk, dv = ring_attn_backward(ring, q, k, v, o, d_o.contiguous(), lse, scale, 0, q.dtype)
         return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), None, None
 
 
