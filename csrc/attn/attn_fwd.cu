@@ -1,15 +1,19 @@
 // Flash-attention forward for sm_100a (head_dim 128, bf16 in, fp32 softmax/accumulate).
 //
 // One CTA owns two adjacent 128-row Q tiles of one head and walks the KV buffer once:
-//   warps 0-7    softmax of BOTH Q tiles, one tile at a time; warp (q, hf) owns 16 TMEM lanes (rows) and reads
-//                them in the accumulator-fragment layout; S/P/O live in TMEM
-//   warp 8       TMA producer: Q once, then K/V tiles through a 2-stage ring (plain per-CTA loads)
-//   warps 9, 10  MMA issuers, one per Q tile: S_i = Q_i K^T (SS form) and O_i += P_i V (A = P read from
-//                TMEM, issued in two halves so that it starts while the softmax finishes the row block)
+//   warps 0-7    softmax, four warps per Q tile, one thread per row, 64 keys at a time; S/P/O live in TMEM
+//   warp 8       TMA producer: Q once, then K/V tiles through a 2-stage ring (plain per-CTA loads); it alone walks
+//                the mask and tells the others which tiles there are
+//   warps 9, 10  MMA issuers, one per Q tile: S_i = Q_i K^T (SS form) and O_i += P_i V (A = P read from TMEM)
 //   warp 11      optional peer pull: copies this CTA's slice of the next ring step's K/V from the owning
 //                GPU into local staging with plain P2P loads while the tiles compute
-// The two Q tiles ping-pong so the tensor core has the other tile's MMAs to run during a softmax.
-// TMEM (512 columns): S0 | S1 | O0 | O1, with the bf16 P_i written over the first half of S_i.
+// TMEM (512 columns): S0 | S1 | O0 | O1; S_i is two halves of 64 keys, each with its bf16 P written over its first
+// half, so that the softmax of one half runs beside the products of the other.
+// Measured, 32 heads over 8 KV heads, causal, in a loop (before -> now): 79 -> 74 us at 16 heads x 4,096 tokens, 562 ->
+// 531 us at 8,192, 8.34 -> 7.82 ms at 32,768; 4,096-token window over 65,536 tokens 5.74 -> 4.68 ms. Before, eight warps
+// served both tiles in turn, 128 keys at a time, every role walked the mask, each tile paid an integer division per
+// warp, and a quarter of the exponentials were polynomials (7.82 -> 8.18 ms when put back: instruction issue and fixed
+// latencies bound the softmax warps now, the special-function unit is busy 57 % of the time, the tensor pipe 70 %).
 // O is only rescaled when a row's running max grew by more than 2^8 (the final 1/l makes the
 // result exact either way). Causal / block-sparse masks come from global token positions, so the
 // same kernel serves plain sequences, zigzag context-parallel shards and every ring step; with
@@ -19,6 +23,7 @@
 #include "../common/tma_host.h"
 #include "attn.h"
 #include "tile_iter.cuh"
+#include "work_order.h"
 
 namespace zx {
 
@@ -29,6 +34,7 @@ constexpr int BQ = 128;
 constexpr int BKV = 128;
 constexpr int TILE_BYTES = BQ * HD * 2;   // 32 KB
 constexpr int HALF_BYTES = TILE_BYTES / 2; // one 64-wide d chunk: 128 rows x 128 B
+constexpr int HALF_KV = 64 * 128;          // 64 rows of a d chunk: start of a tile's second 64 keys
 constexpr int KV_STAGES = 2;
 // Optional in-kernel timeline (compile with -DZX_FWD_TRACE): block 0 stamps the SM clock at the pipeline events
 // of its first 256 KV tiles into a device array that zx_fwd_trace_read() copies out. Not part of normal builds.
@@ -40,10 +46,18 @@ __device__ long long g_fwd_trace[256 * 32];
 #define ZX_TR(slot, iter) do { } while (0)
 #endif
 
-constexpr int TMA_WARP = 8, MMA_WARP0 = 9, MMA_WARP1 = 10, PULL_WARP = 11;
-constexpr int NUM_THREADS = 12 * 32;
+constexpr int TMA_WARP = 16, MMA_WARP0 = 17, MMA_WARP1 = 18, PULL_WARP = 19;
+constexpr int NUM_THREADS = 20 * 32;   // 5 warps per scheduler: 96 registers each
 constexpr int TMEM_COLS = 512;
-constexpr int SMEM_BYTES = 2 * TILE_BYTES + KV_STAGES * 2 * TILE_BYTES + 1024 + 256 + 2 * 2 * 128 * 4;
+constexpr int ITEM_SLOTS = 4;
+constexpr int ITEM_END = -1, ITEM_UNKNOWN = -2;
+constexpr int BAR_BYTES = (20 + 2 * ITEM_SLOTS) * 8 + 2 * ITEM_SLOTS * 8 + 8;
+constexpr int SMEM_BYTES = 2 * TILE_BYTES + KV_STAGES * 2 * TILE_BYTES + 1024 + BAR_BYTES;
+static_assert(KV_STAGES == 2, "items carry one bit of stage");
+// Every FWD_POLY_EVERY-th pair of exponentials on the FMA pipe (exp2_poly2); see above why none by default.
+#ifndef FWD_POLY_EVERY
+#define FWD_POLY_EVERY 1000000
+#endif
 constexpr float NEG_BIG = -1.0e30f;
 constexpr float RESCALE_THRESHOLD = 8.0f;
 
@@ -53,6 +67,7 @@ struct FwdParams {
   int causal, window_blocks, global_every;
   int n_q_tiles, n_kv_tiles;
   int q_tiles_per_chunk, kv_tiles_per_chunk;
+  int heads_per_group;   // block order, see work_order.h
   int q_chunk_pos[kAttnMaxChunks];
   int kv_chunk_pos[kAttnMaxChunks];
   __nv_bfloat16* O;
@@ -73,24 +88,36 @@ __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, ok);
 }
 
+// Warp-uniform bounded wait for a barrier's phase or for *tile to reach m.
+__device__ __forceinline__ bool wait_pv(uint64_t* bar, uint32_t parity, volatile int* tile, int m, volatile int* abort_flag) {
+  const uint64_t t0 = globaltimer_ns();
+#pragma unroll 1
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) || *tile >= m)) return true;
+    if (__any_sync(0xffffffffu, *abort_flag != 0 || globaltimer_ns() - t0 > ZX_WAIT_LIMIT_NS)) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+}
+
 // Rare path of the softmax warps (a row's running maximum grew by more than the threshold): multiply this
 // thread's entries of the output rows by their row's alpha in TMEM (fragment layout: registers 4k, 4k+1 belong
-// to row a, 4k+2, 4k+3 to row b). Kept out of line so that its registers cost the hot loop nothing; the call's
-// register saves only happen when the branch is taken.
-__device__ __noinline__ void rescale_o_rows(uint32_t o_tmem, float alpha_a, float alpha_b) {
+// to row a, 4k+2, 4k+3 to row b). Eight registers at a time and no call: the scores stay in registers meanwhile.
+__device__ __forceinline__ void rescale_o_rows(uint32_t o_tmem, float alpha_a, float alpha_b) {
 #pragma unroll 1
-  for (int c = 0; c < 2; ++c) {
-    uint32_t x[32];
-    tmem_ld_16x256b_x8(o_tmem + c * 64, x);
+  for (int c = 0; c < HD; c += 16) {
+    uint32_t x[8];
+    tmem_ld_16x256b_x2(o_tmem + c, x);
     tmem_wait_ld();
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < 2; ++k) {
       x[4 * k] = __float_as_uint(__uint_as_float(x[4 * k]) * alpha_a);
       x[4 * k + 1] = __float_as_uint(__uint_as_float(x[4 * k + 1]) * alpha_a);
       x[4 * k + 2] = __float_as_uint(__uint_as_float(x[4 * k + 2]) * alpha_b);
       x[4 * k + 3] = __float_as_uint(__uint_as_float(x[4 * k + 3]) * alpha_b);
     }
-    tmem_st_16x256b_x8(o_tmem + c * 64, x);
+    tmem_st_16x256b_x2(o_tmem + c, x);
   }
   tmem_wait_st();
 }
@@ -127,10 +154,10 @@ __device__ __forceinline__ bool dense_allowed(const FwdParams& p, int qpos0, int
 #undef ZX_FWD_SPARSE
 #undef ZX_FWD_KERNEL_NAME
 
-CUtensorMap make_qkv_map(const void* base, int B, int S, int H, int64_t tok_stride) {
+CUtensorMap make_qkv_map(const void* base, int B, int S, int H, int64_t tok_stride, uint32_t rows = 128) {
   uint64_t dims[4] = {(uint64_t)HD, (uint64_t)H, (uint64_t)S, (uint64_t)B};
   uint64_t strides[3] = {(uint64_t)HD * 2, (uint64_t)tok_stride * 2, (uint64_t)S * (uint64_t)tok_stride * 2};
-  uint32_t box[4] = {64, 1, 128, 1};
+  uint32_t box[4] = {64, 1, rows, 1};
   return make_tma_map(base, 2, 4, dims, strides, box, TmaSwizzle::B128);
 }
 
@@ -163,6 +190,7 @@ void launch_attn_fwd(const AttnFwdArgs& a) {
   CUtensorMap tmQ = make_qkv_map(a.q, a.B, a.Sq, a.Hq, a.q_tok_stride);
   CUtensorMap tmK = make_qkv_map(a.k, a.B, a.Skv, a.Hkv, a.k_tok_stride);
   CUtensorMap tmV = make_qkv_map(a.v, a.B, a.Skv, a.Hkv, a.v_tok_stride);
+  CUtensorMap tmO = make_qkv_map(a.o, a.B, a.Sq, a.Hq, (int64_t)a.Hq * HD, 16);   // stored 16 rows at a time
   FwdParams p;
   p.B = a.B; p.Hq = a.Hq; p.Hkv = a.Hkv; p.Sq = a.Sq; p.Skv = a.Skv;
   p.scale_log2 = a.scale * 1.4426950408889634f;
@@ -195,8 +223,14 @@ void launch_attn_fwd(const AttnFwdArgs& a) {
   }
   const int n_pairs = (p.n_q_tiles + 1) / 2;
   const int grid = n_pairs * a.Hq * a.B;
-  if (p.window_blocks > 0) attn_fwd_sparse_kernel<<<grid, NUM_THREADS, SMEM_BYTES, a.stream>>>(tmQ, tmK, tmV, p);
-  else attn_fwd_kernel<<<grid, NUM_THREADS, SMEM_BYTES, a.stream>>>(tmQ, tmK, tmV, p);
+  const bool uniform = !a.mask.causal && a.mask.window_blocks == 0;
+  // a block's longest run is n_pairs steps of two tiles, like the tiles of the rule; whole groups of query heads share
+  // their K and V
+  const int G = a.Hq / a.Hkv;
+  const int per = heads_per_group(n_pairs, a.B * a.Hq, uniform, false);
+  p.heads_per_group = (per + G - 1) / G * G;
+  if (p.window_blocks > 0) attn_fwd_sparse_kernel<<<grid, NUM_THREADS, SMEM_BYTES, a.stream>>>(tmQ, tmK, tmV, tmO, p);
+  else attn_fwd_kernel<<<grid, NUM_THREADS, SMEM_BYTES, a.stream>>>(tmQ, tmK, tmV, tmO, p);
 }
 
 }  // namespace zx

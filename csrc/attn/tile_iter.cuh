@@ -59,7 +59,7 @@ ZX_TI_FN int next_kv_tile(const P& p, int qpos0, int j) {
 }
 
 // Cursor over the KV tiles one Q tile may attend: keeps the chunk of the current tile, so stepping costs
-// no integer division (the forward kernel's MMA warp walks two of these, one per Q tile of its pair).
+// no integer division (the forward kernel's producer walks two of these, one per Q tile of its pair).
 struct KvCursor {
   int j;          // current tile (n_kv_tiles when exhausted)
   int kpos0;      // its first position

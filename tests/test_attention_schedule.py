@@ -55,3 +55,49 @@ def test_attention_backward_writes_every_tile(B, Sq, Skv, Hq, Hkv, causal, wb, g
         # Zero rows: nothing seen, or (window case, row 0) one key, where dP - delta is the difference of two 32-bit sums
         # of 128 products of unit normals, each off by at most 128 * 2^-24 * sum|terms| ~ 1e-3 * 2^-7 ~ 1e-5.
         assert got[ref.abs().amax(-1) == 0].abs().amax().item() <= 1e-5 if (ref.abs().amax(-1) == 0).any() else True
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gain", [1.0, 12.0])
+@pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,causal,wb,ge,qpos,kpos", [
+    (1, 128, 128, 1, 1, True, 0, 0, [0], [0]),              # one Q tile: the second half of the block has nothing to do
+    (2, 384, 640, 2, 1, False, 0, 0, [0], [0]),             # odd tile counts
+    (1, 768, 1536, 2, 2, True, 0, 0, [0, 1152], [0]),       # a pair of Q tiles across two chunks: 3 and 10 KV tiles
+    (1, 768, 768, 2, 1, True, 0, 0, [1152, 0], [768, 0]),   # the other way round, and a tile that sees nothing at first
+    (1, 1280, 1280, 1, 1, True, 2, 4, [0], [0]),            # window and global tiles
+])
+def test_attention_forward_pairs_and_rescaling(B, Sq, Skv, Hq, Hkv, causal, wb, ge, qpos, kpos, gain):
+    """One call, and two calls over the halves of the keys merged, against the fp32 host path. `gain` makes the row maxima
+    grow from tile to tile by more than the 2^8 that the kernel tolerates, so the output is rescaled in flight. Bound:
+    P and V are rounded to bf16 (2^-9), the merged form rounds the output to bf16 twice."""
+    torch.manual_seed(Sq + Skv)
+    mask, scale = MaskSpec(causal, wb, ge), gain / math.sqrt(128)
+    q = torch.randn(B, Sq, Hq, 128).bfloat16()
+    k, v = (torch.randn(B, Skv, Hkv, 128).bfloat16() for _ in range(2))
+    half = Skv // (2 * len(kpos)) * len(kpos) if Skv % (256 * len(kpos)) == 0 else 0
+    results = []
+    for dev in ("cpu", "cuda"):
+        a = [t.to(dev) for t in (q, k, v)]
+        out = []
+        for merge in ([False, True] if half and len(kpos) == 1 else [False]):
+            o = torch.full(q.shape, math.nan, device=dev, dtype=torch.bfloat16)
+            lse = torch.full((B, Hq, Sq), math.nan, device=dev)
+            if merge:
+                lo, hi = ([t[:, part].clone(memory_format=torch.contiguous_format) for t in a[1:]]
+                          for part in (slice(0, half), slice(half, None)))
+                attn_forward(a[0], *hi, o, lse, scale, mask, qpos, [half])
+                attn_forward(a[0], *lo, o, lse, scale, mask, qpos, [0], True)
+            else:
+                attn_forward(*a, o, lse, scale, mask, qpos, kpos)
+            out += [o.float().cpu(), lse.cpu()]
+        results.append(out)
+    _ext.check_status()
+    for n, (ref, got) in enumerate(zip(*results)):
+        if n % 2 == 0:
+            assert torch.isfinite(got).all()
+            assert (got - ref).norm() <= 2e-2 * ref.norm()
+        else:
+            seen = torch.isfinite(ref)
+            assert torch.equal(seen, torch.isfinite(got))
+            # scores are exact products summed in fp32: |s| up to ~60 with the gain, 128 terms, plus the exponentials' 2^-22
+            assert (got[seen] - ref[seen]).abs().max().item() <= 2e-3
