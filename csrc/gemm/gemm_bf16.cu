@@ -1,4 +1,5 @@
-// Persistent bf16 GEMM for sm_100a: C[M,N] = A[M,K] * B[N,K]^T (+ D), fp32 accumulation in TMEM.
+// Persistent bf16 GEMM for sm_100a: C[M,N] = A[M,K] * B[N,K]^T (+ D), fp32 accumulation in TMEM. Two kernels, chosen by
+// shape (choose_tile): CTA pairs with 256 x 256 or 256 x 128 tiles (second half of this file), and single CTAs:
 //
 //  * operands are staged by TMA (128-byte swizzle, per-CTA loads) through a 4-deep mbarrier ring,
 //  * one elected thread issues tcgen05.mma 128x256x16 into one of two 256-column TMEM accumulators,
@@ -44,6 +45,7 @@ struct KParams {
   int d_mode;  // 0: none, 1: bf16 addend, 2: fp32 addend
   int tma_store;  // plain bf16 output: the epilogue goes through shared memory and TMA stores
   int num_m, num_n;
+  int out_mode;   // pair kernel
   const uint4* pull_src;
   uint4* pull_dst;
   size_t pull_nvec;
@@ -52,8 +54,8 @@ struct KParams {
   Status* status;
 };
 
+template <int GM>
 __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& tm, int& tn) {
-  constexpr int GM = 16;
   const int per_group = GM * num_n;
   const int g = t / per_group;
   const int first_m = g * GM;
@@ -119,7 +121,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
         int tm, tn;
-        tile_coords(t, p.num_m, p.num_n, tm, tn);
+        tile_coords<16>(t, p.num_m, p.num_n, tm, tn);
         const int m0 = tm * BM, n0 = tn * BN;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % STAGES;
@@ -206,7 +208,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++lt) {
       int tm, tn;
-      tile_coords(t, p.num_m, p.num_n, tm, tn);
+      tile_coords<16>(t, p.num_m, p.num_n, tm, tn);
       const uint32_t buf = lt & 1;
       if (!mbar_wait(&acc_full[buf], (lt >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
@@ -370,6 +372,267 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// CTA pairs: 256 x 256 or 256 x 128 tiles
+// ------------------------------------------------------------------------------------------
+// Two SMs of a cluster work on one tile (figures for 256 x 256): each holds 128 rows of A and 128 rows of B per k-block (32
+// KB instead of 48 for the same work), the even CTA issues M = 256 MMAs that read both, each CTA keeps 128 rows of the
+// accumulator. That is a third less traffic from L2 and into the tensor cores, and six stages instead of four.
+// Measured (single CTAs -> pairs, three calls / in a loop at the power cap): 16384 x 4096 x 14336 1356 -> 1307 us / 1477 ->
+// 1404; its weight gradient (both operands transposed) 1448 -> 1324 / 1580 -> 1423; 32768 x 28672 x 4096 5268 -> 4996 /
+// 5712 -> 5552; fp32 accumulation 128256 x 4096 x 4096 3682 -> 3067 / 3988 -> 3369 (the reduction in L2 instead of a read
+// by each thread, 16 bytes of 32 rows at a time). cuBLAS: 1210 / 1294 us for the first, 1316 / 1419 for the second.
+// TN: width of the tile, 256 or (for outputs that 256 columns divide badly) 128.
+template <int TN>
+struct PairCfg {
+  static constexpr int B_BYTES = (TN / 2) * BK * 2;             // 16 or 8 KB
+  static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_BYTES;
+  static constexpr int STAGES = 6 * 32768 / STAGE_BYTES;        // 6 or 8: 192 KB
+  static constexpr int SMEM = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+};
+constexpr int PAIR_THREADS = 224;
+static_assert(PairCfg<256>::SMEM <= 227 * 1024 && PairCfg<128>::SMEM <= 227 * 1024, "gemm (pair) shared memory");
+static_assert((2 * PairCfg<128>::STAGES + 9) * 8 + 8 <= 256, "gemm (pair) barriers");
+
+// Output forms of the pair kernel's epilogue; all go through the slabs and the TMA unit.
+constexpr int OUT_BF16 = 0, OUT_BF16_ADD = 1, OUT_FP32 = 2, OUT_FP32_ACC = 3;
+
+template <bool A_MN, bool B_MN, int TN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD, KParams p) {
+  using Cfg = PairCfg<TN>;
+  constexpr int PAIR_STAGES = Cfg::STAGES, PAIR_B_BYTES = Cfg::B_BYTES, PAIR_STAGE_BYTES = Cfg::STAGE_BYTES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sA = smem;                                             // [PAIR_STAGES][16 KB]
+  uint8_t* sB = smem + PAIR_STAGES * A_STAGE_BYTES;               // [PAIR_STAGES][16 or 8 KB]
+  uint8_t* sStage = smem + PAIR_STAGES * PAIR_STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStage + STAGING_BYTES);
+  uint64_t* full = bars;                        // [PAIR_STAGES] even CTA only: both CTAs' tiles of a stage have landed
+  uint64_t* empty = bars + PAIR_STAGES;         // [PAIR_STAGES] each CTA: the MMAs have read the stage
+  uint64_t* acc_full = bars + 2 * PAIR_STAGES;  // [2] each CTA
+  uint64_t* acc_empty = acc_full + 2;           // [2] even CTA only: eight epilogue warps, four of each CTA
+  uint64_t* drain_bar = acc_full + 4;           // 1
+  uint64_t* d_full = acc_full + 5;              // [4] addend slab of epilogue warp q has landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 9);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int num_tiles = p.num_m * p.num_n;      // in 256 x TN tiles
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PAIR_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 8);
+    }
+    mbar_init(drain_bar, 1);
+    for (int w = 0; w < 4; ++w) mbar_init(&d_full[w], 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, 2 * TN);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // the other CTA's barriers exist before anything arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------- TMA producer (both CTAs) -------------------
+    if (lane == 0) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
+      const uint32_t full0 = map_to_cta(full, 0);
+      uint32_t it = 0, ph = 1;
+      int s = 0;
+      bool ok = true;
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step) {
+        int tm, tn;
+        tile_coords<8>(t, p.num_m, p.num_n, tm, tn);
+        const int m0 = tm * 256 + (int)rank * BM, n0 = tn * TN + (int)rank * (TN / 2);
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          if (!mbar_wait(&empty[s], ph, abort_flag)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * PAIR_STAGE_BYTES);
+          uint8_t* a_dst = sA + s * A_STAGE_BYTES;
+          uint8_t* b_dst = sB + s * PAIR_B_BYTES;
+          const uint32_t bar = full0 + 8 * s;
+          if (!A_MN) {
+            tma_load_2d_pair(a_dst, &tmA, bar, kb * BK, m0);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) tma_load_2d_pair(a_dst + c * CHUNK_BYTES, &tmA, bar, m0 + c * 64, kb * BK);
+          }
+          if (!B_MN) {
+            tma_load_2d_pair(b_dst, &tmB, bar, kb * BK, n0);
+          } else {
+#pragma unroll
+            for (int c = 0; c < TN / 128; ++c) tma_load_2d_pair(b_dst + c * CHUNK_BYTES, &tmB, bar, n0 + c * 64, kb * BK);
+          }
+          if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
+        }
+      }
+      if (!ok) {
+        report(p.status, ZX_ERR_TIMEOUT, /*site=*/1, (int)it);
+        const uint64_t t0 = globaltimer_ns();   // loads already issued still land: give them a bounded moment
+        while (globaltimer_ns() - t0 < 2000000ull) {
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------- MMA issuer (even CTA) ----------------------
+    if (rank == 0) {
+      constexpr uint32_t idesc = make_idesc(256, TN, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint64_t a_desc0 = A_MN ? make_smem_desc_sw128(smem_u32(sA), CHUNK_BYTES, 1024)
+                                    : make_smem_desc_sw128(smem_u32(sA), 16, 1024);
+      const uint64_t b_desc0 = B_MN ? make_smem_desc_sw128(smem_u32(sB), CHUNK_BYTES, 1024)
+                                    : make_smem_desc_sw128(smem_u32(sB), 16, 1024);
+      uint32_t it = 0, lt = 0, ph = 0;
+      int s = 0;
+      bool ok = true;
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step, ++lt) {
+        const uint32_t buf = lt & 1;
+        if (!mbar_wait_cluster_w(&acc_empty[buf], ((lt >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * TN;
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          if (!mbar_wait_w(&full[s], ph, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t a_base = desc_advance(a_desc0, (uint32_t)s * A_STAGE_BYTES);
+          const uint64_t b_base = desc_advance(b_desc0, (uint32_t)s * PAIR_B_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_ss_pair_w(d_tmem, desc_advance(a_base, A_MN ? k * UMMA_K * 128 : k * UMMA_K * 2),
+                           desc_advance(b_base, B_MN ? k * UMMA_K * 128 : k * UMMA_K * 2), idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit_pair_w(&empty[s], 3);
+          if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
+        }
+        if (ok) umma_commit_pair_w(&acc_full[buf], 3);
+      }
+      if (!ok) {
+        if (lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/2, (int)it);
+        umma_commit_pair_w(drain_bar, 1);
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 50000000ull) {
+        }
+      }
+    }
+  } else if (warp == W_PULL) {
+    // ------------------------------- peer pull ----------------------------------
+    warp_pull_slice<16>(p.pull_src, p.pull_dst, p.pull_nvec, lane);
+  } else {
+    // ------------------------------- epilogue warps (both CTAs) -----------------
+    const int q = warp & 3;  // TMEM lane quarter this warp may read
+    uint8_t* slabs = sStage + q * 2 * SLAB_BYTES;
+    const uint32_t acc_empty0 = map_to_cta(acc_empty, 0);
+    const bool fp32 = p.out_mode >= OUT_FP32;
+    const int slab_cols = fp32 ? 32 : 64;    // 128 bytes of a row
+    uint32_t lt = 0;
+    uint32_t d_phase = 0;    // parity of this warp's addend barrier
+    uint32_t use = 0;        // slabs used so far
+    bool ok = true;
+    for (int t = first_tile; t < num_tiles && ok; t += tile_step, ++lt) {
+      int tm, tn;
+      tile_coords<8>(t, p.num_m, p.num_n, tm, tn);
+      const uint32_t buf = lt & 1;
+      if (!mbar_wait(&acc_full[buf], (lt >> 1) & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      const int row0 = tm * 256 + (int)rank * BM + q * 32;
+      if (row0 < p.M) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < TN; c0 += slab_cols) {
+          const int col0 = tn * TN + c0;
+          if (col0 >= p.N) break;
+          uint8_t* slab = slabs + (use++ & 1) * SLAB_BYTES;
+          if (lane == 0) {
+            tma_store_wait_read<1>();   // the store that read this slab two chunks ago is done with it
+            if (p.out_mode == OUT_BF16_ADD) {
+              mbar_expect_tx(&d_full[q], SLAB_BYTES);
+              tma_load_2d(slab, &tmD, &d_full[q], col0, row0);
+            }
+          }
+          __syncwarp();   // lane 0 has seen the slab free
+          uint8_t* srow = slab + lane * 128;
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(tmem_addr(tmem_base, q * 32, buf * TN + c0), r);
+          tmem_wait_ld();
+          if (fp32) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<uint4*>(srow + ((c ^ (lane & 7)) << 4)) = make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (h == 1) {
+                tmem_ld_32x32b_x32(tmem_addr(tmem_base, q * 32, buf * TN + c0 + 32), r);
+                tmem_wait_ld();
+              } else if (p.out_mode == OUT_BF16_ADD) {
+                if (!mbar_wait(&d_full[q], d_phase, abort_flag)) { ok = false; break; }
+                d_phase ^= 1u;
+              }
+#pragma unroll
+              for (int c4 = 0; c4 < 4; ++c4) {
+                uint4* cell = reinterpret_cast<uint4*>(srow + (((h * 4 + c4) ^ (lane & 7)) << 4));
+                float2 f[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                  f[e] = make_float2(__uint_as_float(r[8 * c4 + 2 * e]), __uint_as_float(r[8 * c4 + 2 * e + 1]));
+                if (p.out_mode == OUT_BF16_ADD) {   // fp32 accumulator + addend, rounded to bf16 once
+                  const uint4 d = *cell;
+                  const uint32_t dw[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const float2 a = unpack_bf16x2(dw[e]);
+                    f[e].x += a.x;
+                    f[e].y += a.y;
+                  }
+                }
+                *cell = make_uint4(pack_bf16x2(f[0].x, f[0].y), pack_bf16x2(f[1].x, f[1].y), pack_bf16x2(f[2].x, f[2].y),
+                                   pack_bf16x2(f[3].x, f[3].y));
+              }
+            }
+          }
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            // Accumulation into the output itself: the addition is done where the line is (L2), each element by exactly
+            // one store, so the fp32 result is the one that reading, adding and writing it back would give.
+            if (p.out_mode == OUT_FP32_ACC) tma_reduce_add_2d(&tmC, slab, col0, row0);
+            else tma_store_2d(&tmC, slab, col0, row0);
+            tma_store_commit();
+          }
+        }
+      }
+      if (!ok) break;
+      tc_fence_before();
+      mbar_arrive_warp_cluster(acc_empty0 + 8 * buf);
+    }
+    if (!ok && lane == 0) report(p.status, ZX_ERR_TIMEOUT, /*site=*/3, (int)lt);
+    if (lane == 0) tma_store_wait<0>();   // shared memory must outlive the stores that read it
+  }
+
+  // ------------------------------- teardown -------------------------------------
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // neither CTA leaves while the other may still arrive on its barriers or read its tiles
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 2 * TN);
+  }
+}
+
 template <bool A_MN, bool B_MN>
 void launch_variant(const GemmArgs& a, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
                     const CUtensorMap& tmD, const KParams& p, int grid) {
@@ -382,6 +645,66 @@ void launch_variant(const GemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
     configured = true;
   }
   kern<<<grid, NUM_THREADS, SMEM_BYTES, a.stream>>>(tmA, tmB, tmC, tmD, p);
+}
+
+template <bool A_MN, bool B_MN, int TN>
+void launch_pair(const GemmArgs& a, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
+                 const CUtensorMap& tmD, const KParams& p) {
+  static PerDeviceOnce once;
+  static int max_clusters[PerDeviceOnce::kMaxDevices] = {0};
+  bool& configured = once.current();
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= PerDeviceOnce::kMaxDevices) dev = 0;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, TN>;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<TN>::SMEM);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("gemm: cannot raise shared memory limit: ") + cudaGetErrorString(e));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (unsigned)a.sm_count);
+    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.dynamicSmemBytes = PairCfg<TN>::SMEM;
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
+    max_clusters[dev] = e == cudaSuccess && n > 0 ? n : a.sm_count / 2;
+    if (e != cudaSuccess) cudaGetLastError();
+    configured = true;
+  }
+  const int tiles = p.num_m * p.num_n;
+  int clusters = max_clusters[dev] < a.sm_count / 2 ? max_clusters[dev] : a.sm_count / 2;
+  if (clusters > tiles) clusters = tiles;
+  kern<<<2 * clusters, PAIR_THREADS, PairCfg<TN>::SMEM, a.stream>>>(tmA, tmB, tmC, tmD, p);
+}
+
+template <int TN>
+void launch_pair_layout(const GemmArgs& a, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
+                        const CUtensorMap& tmD, const KParams& p) {
+  if (a.a_mn) {
+    if (a.b_mn) launch_pair<true, true, TN>(a, tmA, tmB, tmC, tmD, p);
+    else launch_pair<true, false, TN>(a, tmA, tmB, tmC, tmD, p);
+  } else {
+    if (a.b_mn) launch_pair<false, true, TN>(a, tmA, tmB, tmC, tmD, p);
+    else launch_pair<false, false, TN>(a, tmA, tmB, tmC, tmD, p);
+  }
+}
+
+// Width of the CTA pair's tile, or 0 for the single-CTA kernel: the least of three estimates in microseconds, each launch
+// + waves * (tile + per 1000 of K), with constants fitted to 100 shapes (M 256 to 16384, N 512 to 11264, K 512 to 5640) run
+// with each kernel in turn. Over those shapes the choice costs 0.3 % against the best of the three on average and 4 % at
+// most; the kernels differ by up to 35 %. For example (single / 128 / 256 wide): 256 x 2048 x 4096 22.7 / 18.1 / 23.6 us,
+// 8192 x 2048 x 512 20.6 / 23.2 / 24.2, 3000 x 2056 x 5640 136 / 97 / 108, 4096 x 11264 x 4096 279 / 312 / 238.
+// One row block (M <= 128) leaves half of a pair idle.
+int choose_tile(int M, int N, int K, int sm_count) {
+  if (M <= BM || sm_count < 2) return 0;
+  auto waves = [](int rows, int n_rows, int cols, int n_cols, int units) {
+    const long long tiles = (long long)((rows + n_rows - 1) / n_rows) * ((cols + n_cols - 1) / n_cols);
+    return (double)((tiles + units - 1) / units);
+  };
+  const double k = K * 1e-3;
+  const double single = 2.4 + waves(M, BM, N, BN, sm_count) * (1.8 + 5.1 * k);
+  const double narrow = 4.0 + waves(M, 256, N, 128, sm_count / 2) * (1.1 + 3.2 * k);
+  const double wide = 3.4 + waves(M, 256, N, 256, sm_count / 2) * (1.8 + 4.85 * k);
+  if (single <= wide && single <= narrow) return 0;
+  return wide <= narrow ? 256 : 128;
 }
 
 }  // namespace
@@ -405,20 +728,27 @@ void launch_gemm_bf16(const GemmArgs& a) {
       if (a.scatter_base[r] == nullptr) throw std::runtime_error("gemm_bf16: missing scatter base");
   }
 
+  // a scattered output, and an addend other than these, have their epilogue in the single-CTA kernel
+  const bool acc_self = a.d_mode == 2 && a.out_fp32 && a.D == a.C && a.ldd == a.ldc;
+  const bool pair_form = a.scatter_ranks == 0 && (a.d_mode != 2 || acc_self) && !(a.out_fp32 && a.d_mode == 1);
+  const int tn = pair_form ? choose_tile(a.M, a.N, a.K, a.sm_count) : 0;
+  const bool pair = tn != 0;
+
   // K-major operand: global [rows, K]; box 64 (K) x rows-per-tile.
   // MN-major operand: global [K, rows]; box 64 (rows) x 64 (K), several boxes per stage.
   CUtensorMap tmA = a.a_mn ? make_tma_2d(a.A, 2, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)a.lda, 64, BK)
                            : make_tma_2d(a.A, 2, (uint64_t)a.M, (uint64_t)a.K, (uint64_t)a.lda, BK, BM);
   CUtensorMap tmB = a.b_mn ? make_tma_2d(a.B, 2, (uint64_t)a.K, (uint64_t)a.N, (uint64_t)a.ldb, 64, BK)
-                           : make_tma_2d(a.B, 2, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)a.ldb, BK, BN);
+                           : make_tma_2d(a.B, 2, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)a.ldb, BK, pair ? tn / 2 : BN);
   KParams p;
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.ldc = a.ldc; p.ldd = a.ldd;
   p.C = a.C; p.D = a.D;
   p.out_fp32 = a.out_fp32; p.d_mode = a.d_mode;
   p.tma_store = (!a.out_fp32 && a.d_mode != 2 && a.scatter_ranks == 0) ? 1 : 0;
-  // box: 64 columns (one 128-byte swizzle span) x the 32 rows of one epilogue warp
-  CUtensorMap tmC = p.tma_store ? make_tma_2d(a.C, 2, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldc, 64, 32) : tmA;
+  // box: 128 bytes of columns (one swizzle span) x the 32 rows of one epilogue warp
+  CUtensorMap tmC = pair && a.out_fp32 ? make_tma_2d(a.C, 4, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldc, 32, 32)
+                    : p.tma_store ? make_tma_2d(a.C, 2, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldc, 64, 32) : tmA;
   CUtensorMap tmD = (p.tma_store && a.d_mode == 1) ? make_tma_2d(a.D, 2, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldd, 64, 32) : tmA;
   p.num_m = (a.M + BM - 1) / BM;
   p.num_n = (a.N + BN - 1) / BN;
@@ -430,6 +760,15 @@ void launch_gemm_bf16(const GemmArgs& a) {
   p.scatter_src_rank = a.scatter_src_rank;
   for (int r = 0; r < 8; ++r) p.scatter_base[r] = reinterpret_cast<__nv_bfloat16*>(a.scatter_base[r]);
   p.status = a.status;
+  if (pair) {
+    p.num_m = (a.M + 255) / 256;
+    p.num_n = (a.N + tn - 1) / tn;
+    p.out_mode = a.out_fp32 ? (acc_self ? OUT_FP32_ACC : OUT_FP32) : (a.d_mode == 1 ? OUT_BF16_ADD : OUT_BF16);
+    if (tn == 256) launch_pair_layout<256>(a, tmA, tmB, tmC, tmD, p);
+    else launch_pair_layout<128>(a, tmA, tmB, tmC, tmD, p);
+    return;
+  }
+  p.out_mode = OUT_BF16;
   const int tiles = p.num_m * p.num_n;
   const int grid = tiles < a.sm_count ? tiles : a.sm_count;
   if (a.a_mn) {
