@@ -25,6 +25,7 @@
 #include "../common/device_once.h"
 #include "../common/tma_host.h"
 #include "attn.h"
+#include "dkdv_waits.h"
 #include "tile_iter.cuh"
 #include "work_order.h"
 
@@ -473,8 +474,15 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const bool has_next = n + 1 < n_items;
         const int s_first = scores ? qsn : dsn, s_second = scores ? ds : qs;
         for (int h = 0; h < 2; ++h) {
-          const bool got = h == 0 && has_next ? mbar_wait2_w(&in_ready[0], n & 1, &x_full[s_first], scores ? qphn : dphn, abort_flag)
-                                              : mbar_wait_w(&in_ready[h], n & 1, abort_flag);
+          // what each wait covers: dkdv_waits.h
+          const unsigned waits = dkdv_waits(scores, h, has_next);
+          const bool next = waits & WAIT_NEXT, tile = waits & WAIT_TILE;
+          uint64_t* in = &in_ready[h];
+          const uint32_t par = n & 1;
+          const bool got = waits == WAIT_IN
+                               ? mbar_wait_w(in, par, abort_flag)
+                               : mbar_wait3_w(in, par, next ? &x_full[s_first] : in, next ? (scores ? qphn : dphn) : par,
+                                              tile ? &do_full[ds] : in, tile ? (n >> 1) & 1 : par, abort_flag);
           if (!got) { ok = false; break; }
           tc_fence_after();
           second(h, s_second, (n > 0 || h > 0) ? 1u : 0u);

@@ -179,6 +179,12 @@ __device__ __forceinline__ bool mbar_wait2_w(uint64_t* a, uint32_t pa, uint64_t*
   if (__all_sync(0xffffffffu, ra && rb)) return true;
   return mbar_wait_w(a, pa, abort_flag) && mbar_wait_w(b, pb, abort_flag);
 }
+__device__ __forceinline__ bool mbar_wait3_w(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, uint64_t* c, uint32_t pc,
+                                             volatile int* abort_flag) {
+  const bool ra = mbar_try_wait(a, pa), rb = mbar_try_wait(b, pb), rc = mbar_try_wait(c, pc);
+  if (__all_sync(0xffffffffu, ra && rb && rc)) return true;
+  return mbar_wait_w(a, pa, abort_flag) && mbar_wait_w(b, pb, abort_flag) && mbar_wait_w(c, pc, abort_flag);
+}
 
 // ----------------------------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies). Every load targets the issuing CTA only.

@@ -6,6 +6,7 @@
 
 #include "cpu_ref/flash_cpu.h"
 #include "cpu_ref/quant_adamw_ref.h"
+#include "attn/dkdv_waits.h"
 #include "attn/tile_iter_host.h"
 #include "attn/work_order.h"
 #include "peer/barrier_model.h"
@@ -81,6 +82,7 @@ PYBIND11_MODULE(_host, m) {
     }
     return std::make_pair(per, order);
   }, py::arg("n_tiles"), py::arg("n_heads"), py::arg("longest"), py::arg("uniform"), py::arg("all"));
+  m.def("dkdv_waits", &zx::dkdv_waits, py::arg("scores"), py::arg("h"), py::arg("has_next"));
   m.def("tile_iter_mismatches", &zx::tile_iter_mismatches, py::arg("causal"), py::arg("window_blocks"),
         py::arg("global_every"), py::arg("q_chunk_pos"), py::arg("kv_chunk_pos"), py::arg("q_tiles_per_chunk"),
         py::arg("kv_tiles_per_chunk"));
