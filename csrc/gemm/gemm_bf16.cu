@@ -205,6 +205,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     uint32_t lt = 0;
     uint32_t d_phase = 0;    // parity of this warp's addend barrier
+    uint32_t use = 0;        // slabs used so far, over all tiles: a ragged tile can end after an odd number of chunks
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++lt) {
       int tm, tn;
@@ -228,7 +229,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int cc = 0; cc < BN / 64; ++cc) {
             const int col0 = tn * BN + cc * 64;
             if (col0 >= p.N) break;
-            uint8_t* slab = slabs + (cc & 1) * SLAB_BYTES;
+            uint8_t* slab = slabs + (use++ & 1) * SLAB_BYTES;
             if (lane == 0) {
               tma_store_wait_read<1>();   // the store that read this slab two chunks ago is done with it
               if (p.d_mode == 1) {

@@ -1,4 +1,4 @@
-"""The CTA-pair GEMM at the edges of its tiles, in every operand layout and output form."""
+"""The GEMM kernels at the edges of their tiles, in every operand layout and output form."""
 import pytest
 import torch
 
@@ -42,3 +42,27 @@ def test_pair_gemm_matches_fp64_in_every_form(M, N, K, a_t, b_t):
     close(run(view), ref, 1e-5)
     assert (big[:8] == 7).all() and (big[M + 8:] == 7).all() and (big[:, :32] == 7).all() and (big[:, N + 32:] == 7).all()
     _ext.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("addend", [False, True])
+@pytest.mark.parametrize("N", [2080, 2208])   # the last tile of a row ends after one, after three of four 64-column chunks
+@pytest.mark.parametrize("K", [8, 64])        # short: the next tile's accumulator is ready at once
+def test_single_cta_epilogue_keeps_its_staging_slabs_apart(N, K, addend):
+    """576 single-CTA tiles, so blocks go from a ragged tile to the next one: a slab may only be written again when the
+    store that reads it is done. Bits must repeat, and match fp64 within the rounding to bf16 (2^-9 of the norm at most)."""
+    torch.manual_seed(N + K)
+    M = 8192
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    d = torch.randn(M, N, device="cuda").bfloat16() if addend else None
+    ref = a.double() @ b.double().t() + (d.double() if addend else 0)
+    runs = []
+    for _ in range(8):
+        out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+        _ext.C().gemm(a, b, out, False, False, d)
+        runs.append(out)
+    _ext.check_status()
+    assert all(torch.equal(runs[0], r) for r in runs[1:])
+    # every element: half a unit in the last place of bf16, and the fp32 sum of K + 1 terms of magnitude up to ~30
+    assert ((runs[0].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
