@@ -211,7 +211,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int tm, tn;
       tile_coords<16>(t, p.num_m, p.num_n, tm, tn);
       const uint32_t buf = lt & 1;
-      if (!mbar_wait(&acc_full[buf], (lt >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_w(&acc_full[buf], (lt >> 1) & 1, abort_flag)) { ok = false; break; }   // one verdict for the warp
       tc_fence_after();
       const int row = tm * BM + q * 32 + lane;
       const bool row_ok = row < p.M;
@@ -246,7 +246,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               tmem_wait_ld();
               if (p.d_mode == 1) {
                 if (h == 0) {
-                  if (!mbar_wait(&d_full[q], d_phase, abort_flag)) { ok = false; break; }
+                  if (!mbar_wait_w(&d_full[q], d_phase, abort_flag)) { ok = false; break; }
                   d_phase ^= 1u;
                 }
 #pragma unroll
@@ -547,7 +547,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int tm, tn;
       tile_coords<8>(t, p.num_m, p.num_n, tm, tn);
       const uint32_t buf = lt & 1;
-      if (!mbar_wait(&acc_full[buf], (lt >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_w(&acc_full[buf], (lt >> 1) & 1, abort_flag)) { ok = false; break; }   // one verdict for the warp
       tc_fence_after();
       const int row0 = tm * 256 + (int)rank * BM + q * 32;
       if (row0 < p.M) {
@@ -579,7 +579,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                 tmem_ld_32x32b_x32(tmem_addr(tmem_base, q * 32, buf * TN + c0 + 32), r);
                 tmem_wait_ld();
               } else if (p.out_mode == OUT_BF16_ADD) {
-                if (!mbar_wait(&d_full[q], d_phase, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_w(&d_full[q], d_phase, abort_flag)) { ok = false; break; }
                 d_phase ^= 1u;
               }
 #pragma unroll
@@ -604,7 +604,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               }
             }
           }
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          if (!ok) break;
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
