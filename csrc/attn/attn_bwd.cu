@@ -230,8 +230,10 @@ __device__ __forceinline__ uint64_t base_mnmajor(uint32_t tile_addr) {
 // delta[b, h, s] = sum_d dO * O
 // ------------------------------------------------------------------------------------------
 // Bound by memory: one warp takes eight consecutive tokens of one head (two 256-byte rows per load instruction, all
-// eight loads of a lane in flight, eight neighbouring results per store).
+// eight loads of a lane in flight, eight neighbouring results per store). O_VEC: 16-byte loads of o, or two of 8 bytes for
+// an o that starts in the middle of a 16-byte unit (d_o is also read by TMA, which takes whole units only).
 constexpr int DELTA_TOKENS = 8;
+template <typename O_VEC>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
                                                          const __nv_bfloat16* __restrict__ d_o,
                                                          float* __restrict__ delta, int S, int H, int n_groups) {
@@ -244,7 +246,12 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const size_t off = (row0 + (size_t)2 * i * H) * (HD / 8) + (lane & 15);
-    a[i] = __ldg(reinterpret_cast<const uint4*>(o) + off);
+    if constexpr (sizeof(O_VEC) == 16) {
+      a[i] = __ldg(reinterpret_cast<const uint4*>(o) + off);
+    } else {
+      const uint2 lo = __ldg(reinterpret_cast<const uint2*>(o) + 2 * off), hi = __ldg(reinterpret_cast<const uint2*>(o) + 2 * off + 1);
+      a[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+    }
     g[i] = __ldg(reinterpret_cast<const uint4*>(d_o) + off);
   }
   float out = 0.f;
@@ -1002,11 +1009,9 @@ void set_smem(K kern, int bytes, const char* name) {
 void launch_attn_bwd(const AttnBwdArgs& a) {
   check_attn_common(a.Hq, a.Hkv, a.Sq, a.Skv, a.q_layout, a.kv_layout);
   if (a.Sq == 0 || a.Skv == 0 || a.B == 0) return;
-  if (a.compute_delta) {
-    const int groups = (int)((size_t)a.B * a.Sq * a.Hq / DELTA_TOKENS);
-    attn_delta_kernel<<<(groups + 7) / 8, 256, 0, a.stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.delta,
-                                                              a.Sq, a.Hq, groups);
-  }
+  // everything that can refuse the call comes before the first launch
+  const uintptr_t o_align = reinterpret_cast<uintptr_t>(a.o);
+  if (a.compute_delta && o_align % 8 != 0) throw std::runtime_error("attn_bwd: o must be 8-byte aligned");
   CUtensorMap tmQ = make_qkv_map(a.q, a.B, a.Sq, a.Hq, a.q_tok_stride);
   CUtensorMap tmdO = make_qkv_map(a.d_o, a.B, a.Sq, a.Hq, (int64_t)a.Hq * HD);
   CUtensorMap tmK = make_qkv_map(a.k, a.B, a.Skv, a.Hkv, a.k_tok_stride);
@@ -1053,6 +1058,12 @@ void launch_attn_bwd(const AttnBwdArgs& a) {
   p.kv_heads_per_group = heads_per_group(p.n_q_tiles, a.B * a.Hkv, uniform, a.mask.window_blocks > 0);
   p.q_heads_per_group = heads_per_group(p.n_kv_tiles, a.B * a.Hq, uniform, false);
   const unsigned grid_kv = p.n_kv_tiles * a.B * a.Hkv, grid_q = p.n_q_tiles * a.B * a.Hq;
+  if (a.compute_delta) {
+    const int groups = (int)((size_t)a.B * a.Sq * a.Hq / DELTA_TOKENS);
+    auto delta = o_align % 16 == 0 ? attn_delta_kernel<uint4> : attn_delta_kernel<uint2>;
+    delta<<<(groups + 7) / 8, 256, 0, a.stream>>>((const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.delta, a.Sq, a.Hq,
+                                                  groups);
+  }
   if (p.window_blocks > 0) {
     attn_bwd_dkdv_kernel<true><<<grid_kv, DKDV_THREADS, DKDV_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, tmGK, tmGV, p);
     attn_bwd_dq_kernel<true><<<grid_q, DQ_THREADS, DQ_SMEM, a.stream>>>(tmQ, tmdO, tmK, tmV, tmGQ, p);

@@ -101,3 +101,42 @@ def test_attention_forward_pairs_and_rescaling(B, Sq, Skv, Hq, Hkv, causal, wb, 
             assert torch.equal(seen, torch.isfinite(got))
             # scores are exact products summed in fp32: |s| up to ~60 with the gain, 128 terms, plus the exponentials' 2^-22
             assert (got[seen] - ref[seen]).abs().max().item() <= 2e-3
+
+
+def _shifted(t, elements):
+    """A contiguous copy of t that starts `elements` elements into a 16-byte unit."""
+    buf = torch.empty(t.numel() + 8, device=t.device, dtype=t.dtype)
+    out = buf[elements: elements + t.numel()].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+@pytest.mark.gpu
+def test_attention_backward_takes_o_at_8_bytes_and_refuses_before_it_launches():
+    """o is read by the delta pre-pass alone, 8 bytes of it at the least; d_o by TMA too, which takes 16-byte units."""
+    torch.manual_seed(5)
+    B, S, Hq, Hkv, scale = 2, 256, 4, 2, 1.0 / math.sqrt(128)
+    q, do = (torch.randn(B, S, Hq, 128, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, S, Hkv, 128, device="cuda").bfloat16() for _ in range(2))
+    o, lse = torch.empty_like(q), torch.empty(B, Hq, S, device="cuda")
+    attn_forward(q, k, v, o, lse, scale, MaskSpec(), [0], [0])
+
+    def backward(o, do):
+        delta = torch.full_like(lse, 7.0)
+        grads = [torch.full(t.shape, 7.0, device="cuda") for t in (q, k, v)]
+        try:
+            attn_backward(q, k, v, o, do, lse, delta, *grads, scale, MaskSpec(), [0], [0], kv_overwrite=True)
+        except RuntimeError as e:
+            assert "aligned" in str(e)
+            assert all((t == 7.0).all() for t in (delta, *grads))   # nothing ran
+            return None
+        return (delta, *grads)
+
+    want = backward(o, do)
+    got = backward(_shifted(o, 4), do)
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    for elements in (1, 2):
+        assert backward(_shifted(o, elements), do) is None
+    for elements in (1, 4):
+        assert backward(o, _shifted(do, elements)) is None
+    _ext.check_status()
