@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from zenyx_b200.ops import _ext
-from zenyx_b200.ops.attention import MaskSpec, attn_backward, attn_forward
+from zenyx_b200.ops.attention import MaskSpec, attn_backward, attn_forward, flash_attention, ring_flash_attention
 
 
 @pytest.mark.parametrize("n_tiles", [1, 2, 3, 17, 64, 256, 300])
@@ -140,3 +140,15 @@ def test_attention_backward_takes_o_at_8_bytes_and_refuses_before_it_launches():
     for elements in (1, 4):
         assert backward(o, _shifted(do, elements)) is None
     _ext.check_status()
+
+
+def test_gradients_of_mixed_types_are_rounded_to_each_input_s_own():
+    """A ring of one rank on the CPU takes q, k and v of different types; fp32 gradients are not rounded to q's type."""
+    torch.manual_seed(6)
+    q = torch.randn(1, 128, 2, 128).bfloat16().requires_grad_(True)
+    k, v = (torch.randn(1, 128, 1, 128).requires_grad_(True) for _ in range(2))
+    do = torch.randn(1, 128, 2, 128).bfloat16()
+    got = torch.autograd.grad(ring_flash_attention(q, k, v), (q, k, v), do)
+    want = torch.autograd.grad(flash_attention(q, k, v), (q, k, v), do)
+    assert [g.dtype for g in got] == [torch.bfloat16, torch.float32, torch.float32]
+    assert all(torch.equal(a, b) for a, b in zip(got, want))

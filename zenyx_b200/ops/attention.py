@@ -356,14 +356,14 @@ def ring_attn_forward(ctx: RingContext, q, k, v, scale: float, slot: int = 0):
 
 
 def ring_attn_backward(ctx: RingContext, q, k, v, o, d_o, lse, scale: float, slot: int = 0,
-                       grad_dtype: torch.dtype = torch.float32):
+                       grad_dtype: Optional[torch.dtype] = torch.float32):
     """Backward over all ring steps. Returns (dq fp32, dk fp32, dv fp32) for this rank's tokens;
     on GPU dk/dv are views of this rank's peer-visible accumulators (valid until the slot is reused).
-    ``grad_dtype`` is what a ring of one rank, which adds nothing up, returns them in."""
+    ``grad_dtype`` is what a ring of one rank, which adds nothing up, returns them in (None: each in its input's type)."""
     B, Sq, Hq, D = q.shape
     delta = torch.empty_like(lse)
     if ctx.degree == 1:
-        dq, dk, dv = (torch.empty(t.shape, device=t.device, dtype=grad_dtype) for t in (q, k, v))
+        dq, dk, dv = (torch.empty(t.shape, device=t.device, dtype=grad_dtype or t.dtype) for t in (q, k, v))
         attn_backward(q, k, v, o, d_o, lse, delta, dq, dk, dv, scale, ctx.mask, ctx.positions(), ctx.positions(),
                       kv_overwrite=True)
         return dq, dk, dv
@@ -438,7 +438,7 @@ class _RingAttnFn(torch.autograd.Function):
             ks.copy_(k)
             vs.copy_(v)
             k, v = ks, vs
-        dq, dk, dv = ring_attn_backward(ring, q, k, v, o, d_o.contiguous(), lse, scale, 0, q.dtype)
+        dq, dk, dv = ring_attn_backward(ring, q, k, v, o, d_o.contiguous(), lse, scale, 0, None)
         return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), None, None
 
 
