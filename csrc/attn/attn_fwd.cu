@@ -39,9 +39,19 @@ constexpr int KV_STAGES = 2;
 // Optional in-kernel timeline (compile with -DZX_FWD_TRACE): block 0 stamps the SM clock at the pipeline events
 // of its first 256 KV tiles into a device array that zx_fwd_trace_read() copies out. Not part of normal builds.
 #ifdef ZX_FWD_TRACE
-__device__ long long g_fwd_trace[256 * 32];
-#define ZX_TR(slot, iter) \
-  do { if (blockIdx.x == 0 && lane == 0 && (iter) < 256u) g_fwd_trace[(iter) * 32 + (slot)] = clock64(); } while (0)
+// Slots of an iteration: when a softmax warp has its scores, when it has written its probabilities, steps of the issuing warps.
+constexpr int TRACE_ITERS = 256, TRACE_SLOTS = 72;
+constexpr int tr_scores(int half, int warp) { return 16 * half + warp; }
+constexpr int tr_probs(int half, int warp) { return 32 + 16 * half + warp; }
+constexpr int tr_mma(int tile, int step) { return 64 + 4 * tile + step; }
+static_assert(tr_scores(1, 15) < tr_probs(0, 0) && tr_probs(1, 15) < tr_mma(0, 0) && tr_mma(1, 3) < TRACE_SLOTS,
+              "every stamp has a slot of its own");
+__device__ long long g_fwd_trace[TRACE_ITERS * TRACE_SLOTS];
+#define ZX_TR(slot, iter)                                                                             \
+  do {                                                                                                \
+    if (blockIdx.x == 0 && lane == 0 && (iter) < (uint32_t)TRACE_ITERS)                               \
+      g_fwd_trace[(iter) * TRACE_SLOTS + (slot)] = clock64();                                         \
+  } while (0)
 #else
 #define ZX_TR(slot, iter) do { } while (0)
 #endif
@@ -165,7 +175,7 @@ CUtensorMap make_qkv_map(const void* base, int B, int S, int H, int64_t tok_stri
 
 #ifdef ZX_FWD_TRACE
 extern "C" int zx_fwd_trace_read(long long* host_dst) {
-  return (int)cudaMemcpyFromSymbol(host_dst, g_fwd_trace, sizeof(long long) * 256 * 32);
+  return (int)cudaMemcpyFromSymbol(host_dst, g_fwd_trace, sizeof(long long) * TRACE_ITERS * TRACE_SLOTS);
 }
 #endif
 
