@@ -41,9 +41,9 @@ constexpr int KV_STAGES = 2;
 #ifdef ZX_FWD_TRACE
 // Slots of an iteration: when a softmax warp has its scores, when it has written its probabilities, steps of the issuing warps.
 constexpr int TRACE_ITERS = 256, TRACE_SLOTS = 72;
-constexpr int tr_scores(int half, int warp) { return 16 * half + warp; }
-constexpr int tr_probs(int half, int warp) { return 32 + 16 * half + warp; }
-constexpr int tr_mma(int tile, int step) { return 64 + 4 * tile + step; }
+__host__ __device__ constexpr int tr_scores(int half, int warp) { return 16 * half + warp; }
+__host__ __device__ constexpr int tr_probs(int half, int warp) { return 32 + 16 * half + warp; }
+__host__ __device__ constexpr int tr_mma(int tile, int step) { return 64 + 4 * tile + step; }
 static_assert(tr_scores(1, 15) < tr_probs(0, 0) && tr_probs(1, 15) < tr_mma(0, 0) && tr_mma(1, 3) < TRACE_SLOTS,
               "every stamp has a slot of its own");
 __device__ long long g_fwd_trace[TRACE_ITERS * TRACE_SLOTS];
