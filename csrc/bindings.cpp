@@ -64,7 +64,7 @@ std::vector<int64_t> read_status(bool clear) {
 //   a: [M,K] (a_t=false) or [K,M] (a_t=true); b: [N,K] (b_t=false) or [K,N] (b_t=true)
 void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_t, bool b_t, const c10::optional<Tensor>& addend,
           int64_t pull_src, int64_t pull_dst, int64_t pull_bytes, const std::vector<int64_t>& scatter_ptrs,
-          int64_t scatter_rows_per_rank, int64_t scatter_src_rank) {
+          int64_t scatter_rows_per_rank, int64_t scatter_src_rank, int64_t tile) {
   check_bf16(a, "a");
   check_bf16(b, "b");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2, "gemm expects matrices");
@@ -116,6 +116,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_t, bool b_t, con
   g.status = status_ptr();
   g.stream = cur_stream();
   g.sm_count = sm_count();
+  g.tile = (int)tile;
   zx::launch_gemm_bf16(g);
   check_launch("gemm");
 }
@@ -513,7 +514,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("read_status", &read_status, "read (and optionally clear) the kernel status word");
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("a_t"), py::arg("b_t"), py::arg("addend"),
         py::arg("pull_src") = 0, py::arg("pull_dst") = 0, py::arg("pull_bytes") = 0,
-        py::arg("scatter_ptrs") = std::vector<int64_t>{}, py::arg("scatter_rows_per_rank") = 0, py::arg("scatter_src_rank") = 0);
+        py::arg("scatter_ptrs") = std::vector<int64_t>{}, py::arg("scatter_rows_per_rank") = 0, py::arg("scatter_src_rank") = 0,
+        py::arg("tile") = -1);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("d_o"), py::arg("lse"),
         py::arg("delta"), py::arg("dq"), py::arg("dk"), py::arg("dv"), py::arg("scale"), py::arg("causal"),

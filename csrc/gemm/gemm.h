@@ -37,6 +37,7 @@ struct GemmArgs {
   Status* status = nullptr;
   cudaStream_t stream = nullptr;
   int sm_count = 148;
+  int tile = -1;  // -1: tile_choice.h decides; 0 (single CTAs), 128, 256: that kernel, for tests and for fitting the rule
 };
 
 void launch_gemm_bf16(const GemmArgs& args);

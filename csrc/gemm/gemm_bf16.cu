@@ -1,5 +1,5 @@
 // Persistent bf16 GEMM for sm_100a: C[M,N] = A[M,K] * B[N,K]^T (+ D), fp32 accumulation in TMEM. Two kernels, chosen by
-// shape (choose_tile): CTA pairs with 256 x 256 or 256 x 128 tiles (second half of this file), and single CTAs:
+// shape (gemm_choose_tile): CTA pairs with 256 x 256 or 256 x 128 tiles (second half of this file), and single CTAs:
 //
 //  * operands are staged by TMA (128-byte swizzle, per-CTA loads) through a 4-deep mbarrier ring,
 //  * one elected thread issues tcgen05.mma 128x256x16 into one of two 256-column TMEM accumulators,
@@ -13,6 +13,7 @@
 #include "../common/device_once.h"
 #include "../common/tma_host.h"
 #include "gemm.h"
+#include "tile_choice.h"
 
 namespace zx {
 
@@ -609,7 +610,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           __syncwarp();
           if (lane == 0) {
             // Accumulation into the output itself: the addition is done where the line is (L2), each element by exactly
-            // one store, so the fp32 result is the one that reading, adding and writing it back would give.
+            // one store, so the fp32 result is the one that reading, adding and writing it back gives (subnormal operands
+            // and results are zero in both: the reduction flushes them, and so does -ftz in the single-CTA kernel).
             if (p.out_mode == OUT_FP32_ACC) tma_reduce_add_2d(&tmC, slab, col0, row0);
             else tma_store_2d(&tmC, slab, col0, row0);
             tma_store_commit();
@@ -688,26 +690,6 @@ void launch_pair_layout(const GemmArgs& a, const CUtensorMap& tmA, const CUtenso
   }
 }
 
-// Width of the CTA pair's tile, or 0 for the single-CTA kernel: the least of three estimates in microseconds, each launch
-// + waves * (tile + per 1000 of K), with constants fitted to 100 shapes (M 256 to 16384, N 512 to 11264, K 512 to 5640) run
-// with each kernel in turn. Over those shapes the choice costs 0.3 % against the best of the three on average and 4 % at
-// most; the kernels differ by up to 35 %. For example (single / 128 / 256 wide): 256 x 2048 x 4096 22.7 / 18.1 / 23.6 us,
-// 8192 x 2048 x 512 20.6 / 23.2 / 24.2, 3000 x 2056 x 5640 136 / 97 / 108, 4096 x 11264 x 4096 279 / 312 / 238.
-// One row block (M <= 128) leaves half of a pair idle.
-int choose_tile(int M, int N, int K, int sm_count) {
-  if (M <= BM || sm_count < 2) return 0;
-  auto waves = [](int rows, int n_rows, int cols, int n_cols, int units) {
-    const long long tiles = (long long)((rows + n_rows - 1) / n_rows) * ((cols + n_cols - 1) / n_cols);
-    return (double)((tiles + units - 1) / units);
-  };
-  const double k = K * 1e-3;
-  const double single = 2.4 + waves(M, BM, N, BN, sm_count) * (1.8 + 5.1 * k);
-  const double narrow = 4.0 + waves(M, 256, N, 128, sm_count / 2) * (1.1 + 3.2 * k);
-  const double wide = 3.4 + waves(M, 256, N, 256, sm_count / 2) * (1.8 + 4.85 * k);
-  if (single <= wide && single <= narrow) return 0;
-  return wide <= narrow ? 256 : 128;
-}
-
 }  // namespace
 
 void launch_gemm_bf16(const GemmArgs& a) {
@@ -732,7 +714,9 @@ void launch_gemm_bf16(const GemmArgs& a) {
   // a scattered output, and an addend other than these, have their epilogue in the single-CTA kernel
   const bool acc_self = a.d_mode == 2 && a.out_fp32 && a.D == a.C && a.ldd == a.ldc;
   const bool pair_form = a.scatter_ranks == 0 && (a.d_mode != 2 || acc_self) && !(a.out_fp32 && a.d_mode == 1);
-  const int tn = pair_form ? choose_tile(a.M, a.N, a.K, a.sm_count) : 0;
+  const int tn = a.tile >= 0 ? a.tile : pair_form ? gemm_choose_tile(a.M, a.N, a.K, a.sm_count) : 0;
+  if (tn != 0 && ((tn != 128 && tn != 256) || !pair_form || a.sm_count < 2))
+    throw std::runtime_error("gemm_bf16: no kernel of that tile width for this call");
   const bool pair = tn != 0;
 
   // K-major operand: global [rows, K]; box 64 (K) x rows-per-tile.

@@ -9,6 +9,7 @@
 #include "attn/dkdv_waits.h"
 #include "attn/tile_iter_host.h"
 #include "attn/work_order.h"
+#include "gemm/tile_choice.h"
 #include "peer/barrier_model.h"
 #include "tier/belady_min.h"
 #include "tier/tier_engine.h"
@@ -82,6 +83,7 @@ PYBIND11_MODULE(_host, m) {
     }
     return std::make_pair(per, order);
   }, py::arg("n_tiles"), py::arg("n_heads"), py::arg("longest"), py::arg("uniform"), py::arg("all"));
+  m.def("gemm_choose_tile", &zx::gemm_choose_tile, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("sm_count"));
   m.def("dkdv_waits", &zx::dkdv_waits, py::arg("scores"), py::arg("h"), py::arg("has_next"));
   m.def("tile_iter_mismatches", &zx::tile_iter_mismatches, py::arg("causal"), py::arg("window_blocks"),
         py::arg("global_every"), py::arg("q_chunk_pos"), py::arg("kv_chunk_pos"), py::arg("q_tiles_per_chunk"),
