@@ -610,8 +610,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           __syncwarp();
           if (lane == 0) {
             // Accumulation into the output itself: the addition is done where the line is (L2), each element by exactly
-            // one store, so the fp32 result is the one that reading, adding and writing it back gives (subnormal operands
-            // and results are zero in both: the reduction flushes them, and so does -ftz in the single-CTA kernel).
+            // one store, so the fp32 result is the one that reading, adding and writing it back gives. Subnormal operands and
+            // results differ: the single-CTA kernel, built with -ftz, takes them for zero, the reduction keeps them (measured).
             if (p.out_mode == OUT_FP32_ACC) tma_reduce_add_2d(&tmC, slab, col0, row0);
             else tma_store_2d(&tmC, slab, col0, row0);
             tma_store_commit();
