@@ -49,12 +49,21 @@ inline CUtensorMap make_tma_map(const void* base, int elem_bytes, int rank, cons
   CUtensorMapDataType dt = elem_bytes == 2   ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                            : elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                              : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  CUresult r = get_encode_tiled()(&m, dt, (cuuint32_t)rank, const_cast<void*>(base), gdims, gstr, bx, es,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                  swz == TmaSwizzle::B128  ? CU_TENSOR_MAP_SWIZZLE_128B
-                                  : swz == TmaSwizzle::B64 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                           : CU_TENSOR_MAP_SWIZZLE_NONE,
-                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return get_encode_tiled()(&m, dt, (cuuint32_t)rank, const_cast<void*>(base), gdims, gstr, bx, es,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              swz == TmaSwizzle::B128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                              : swz == TmaSwizzle::B64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                       : CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A driver call on a thread that has made no runtime call yet (a thread of the autograd engine whose memory all came
+    // from the allocator's cache): the runtime binds the device's context to a thread only then.
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
   return m;
 }

@@ -701,3 +701,35 @@ def test_checked_build_runs_clean():
     env = dict(os.environ, ZENYX_B200_EXT_DIR=d, PYTHONPATH=os.path.dirname(os.path.dirname(zenyx_b200.__file__)))
     res = subprocess.run([sys.executable, "-c", _CHECKED_SCRIPT], env=env, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0 and "checked ok" in res.stdout, res.stdout[-2000:] + res.stderr[-2000:]
+
+
+def test_first_call_of_a_thread_may_be_a_kernel(C):
+    """Every operation that encodes tensor maps, as the first thing a new thread does: nothing there has touched the CUDA
+    runtime yet (a thread of the autograd engine is in that state while its memory comes from the allocator's cache)."""
+    import threading
+
+    a, b = torch.randn(256, 64, device="cuda").bfloat16(), torch.randn(128, 64, device="cuda").bfloat16()
+    out = torch.empty(256, 128, device="cuda", dtype=torch.bfloat16)
+    q = torch.randn(1, 128, 1, 128, device="cuda").bfloat16()
+    o, lse, delta = torch.empty_like(q), torch.empty(1, 1, 128, device="cuda"), torch.empty(1, 1, 128, device="cuda")
+    dq, dk, dv = (torch.zeros(1, 128, 1, 128, device="cuda") for _ in range(3))
+    errors = []
+
+    def on_a_new_thread(fn):
+        def body():
+            try:
+                fn()
+            except Exception as e:
+                errors.append(repr(e))
+
+        t = threading.Thread(target=body)
+        t.start()
+        t.join()
+
+    on_a_new_thread(lambda: C.gemm(a, b, out, False, False, None))
+    on_a_new_thread(lambda: C.attn_fwd(q, q, q, o, lse, 0.1, True, 0, 0, [0], [0], False, 0, 0, 0))
+    on_a_new_thread(lambda: C.attn_bwd(q, q, q, o, q, lse, delta, dq, dk, dv, 0.1, True, 0, 0, [0], [0], True, False, 0, 0, 0))
+    assert errors == []
+    _status_ok()
+    assert _close(out, a.float() @ b.float().t())
+    assert torch.isfinite(dq).all() and torch.isfinite(dk).all()
