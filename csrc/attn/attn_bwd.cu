@@ -20,6 +20,9 @@
 // full. The dQ kernel has room for Q and dO in TMEM and pays nothing (2,110 -> 1,740 clk per item, MMA time 1,536).
 // Kernel times, 32 heads over 8 KV heads, causal (before -> now): dK/dV 1,140 -> 816 us at 8,192 tokens, 16.2 -> 13.6 ms
 // at 32,768; dQ 709 -> 635 us and 11.0 -> 9.5 ms (the GPU runs at its power cap at 32,768, 1.5 GHz).
+// Exponentials are the special-function unit's: taking every second pair as a polynomial on the FMA pipe made no difference
+// (28.4 -> 29.1 ms for the whole backward at 32,768 tokens at the time), since instruction issue and the cycle of an item
+// bound these kernels.
 // All waits are bounded.
 #include "../common/ptx.cuh"
 #include "../common/device_once.h"
@@ -42,19 +45,6 @@ constexpr int HALF_BYTES = TILE_BYTES / 2; // one 64-wide d chunk
 constexpr int HALF_Q = 64 * 128;           // 64 rows of a d chunk: start of a tile's second half of tokens
 constexpr int TMEM_COLS = 512;
 constexpr float LOG2E = 1.4426950408889634f;
-// Every BWD_POLY_EVERY-th pair of exponentials can be evaluated as a polynomial on the FMA pipe instead of the
-// special-function unit. Measured: these kernels are bound by instruction issue and by their dependency
-// chain, not by that unit, and the polynomial's extra instructions cost as much as they save (29.1 ms with
-// every second pair, 28.4 ms with none at S = 32768), so the default is none.
-#ifndef BWD_POLY_EVERY
-#define BWD_POLY_EVERY 1000000
-#endif
-#ifndef DQ_POLY_EVERY
-#define DQ_POLY_EVERY BWD_POLY_EVERY
-#endif
-#ifndef DKDV_POLY_EVERY
-#define DKDV_POLY_EVERY BWD_POLY_EVERY
-#endif
 
 struct BwdParams {
   int B, Hq, Hkv, Sq, Skv;
@@ -547,7 +537,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             constexpr int c = 2 * c4 + h;
             const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[2 * c]), __uint_as_float(sr[2 * c + 1])), sl2,
                                         h == 0 ? make_float2(nl.x, nl.y) : make_float2(nl.z, nl.w));
-            const float2 e = exp2_pair<c, DKDV_POLY_EVERY>(x);
+            const float2 e = fast_exp2(x);
             sr[2 * c] = __float_as_uint(e.x);
             sr[2 * c + 1] = __float_as_uint(e.y);
           });
@@ -906,7 +896,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         static_for<16>([&](auto idx) {   // packed fp32x2 math: two key columns per instruction
           constexpr int c = decltype(idx)::value;
           const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[2 * c]), __uint_as_float(sr[2 * c + 1])), sl2, nl2);
-          const float2 e = exp2_pair<c, DQ_POLY_EVERY>(x);
+          const float2 e = fast_exp2(x);
           sr[2 * c] = __float_as_uint(e.x);
           sr[2 * c + 1] = __float_as_uint(e.y);
         });

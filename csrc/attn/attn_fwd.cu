@@ -1,11 +1,12 @@
 // Flash-attention forward for sm_100a (head_dim 128, bf16 in, fp32 softmax/accumulate).
 //
 // One CTA owns two adjacent 128-row Q tiles of one head and walks the KV buffer once:
-//   warps 0-7    softmax, four warps per Q tile, one thread per row, 64 keys at a time; S/P/O live in TMEM
-//   warp 8       TMA producer: Q once, then K/V tiles through a 2-stage ring (plain per-CTA loads); it alone walks
+//   warps 0-15   softmax, eight warps per Q tile, 64 keys at a time: a warp has 16 rows, a row lives in four neighbouring
+//                threads; S/P/O live in TMEM
+//   warp 16      TMA producer: Q once, then K/V tiles through a 2-stage ring (plain per-CTA loads); it alone walks
 //                the mask and tells the others which tiles there are
-//   warps 9, 10  MMA issuers, one per Q tile: S_i = Q_i K^T (SS form) and O_i += P_i V (A = P read from TMEM)
-//   warp 11      optional peer pull: copies this CTA's slice of the next ring step's K/V from the owning
+//   warps 17, 18 MMA issuers, one per Q tile: S_i = Q_i K^T (SS form) and O_i += P_i V (A = P read from TMEM)
+//   warp 19      optional peer pull: copies this CTA's slice of the next ring step's K/V from the owning
 //                GPU into local staging with plain P2P loads while the tiles compute
 // TMEM (512 columns): S0 | S1 | O0 | O1; S_i is two halves of 64 keys, each with its bf16 P written over its first
 // half, so that the softmax of one half runs beside the products of the other.
@@ -64,10 +65,6 @@ constexpr int ITEM_END = -1, ITEM_UNKNOWN = -2;
 constexpr int BAR_BYTES = (20 + 2 * ITEM_SLOTS) * 8 + 2 * ITEM_SLOTS * 8 + 8;
 constexpr int SMEM_BYTES = 2 * TILE_BYTES + KV_STAGES * 2 * TILE_BYTES + 1024 + BAR_BYTES;
 static_assert(KV_STAGES == 2, "items carry one bit of stage");
-// Every FWD_POLY_EVERY-th pair of exponentials on the FMA pipe (exp2_poly2); see above why none by default.
-#ifndef FWD_POLY_EVERY
-#define FWD_POLY_EVERY 1000000
-#endif
 constexpr float NEG_BIG = -1.0e30f;
 constexpr float RESCALE_THRESHOLD = 8.0f;
 
