@@ -180,5 +180,6 @@ def test_row_sums_are_rounded_at_their_own_magnitude_once_per_half_tile():
     """131,072 keys: 2,048 halves of 64 keys, whose sums each thread adds to a running sum of its even and one of its odd
     columns. Rounding to nearest at the running value (standard deviation 0.29 * 2^-23.5 of it, on average over its growth
     0.58 of the final one) 2,048 times in each of the eight running sums of a row: 45 * 2.4e-8 * 0.58 / sqrt(8) = 2.2e-7 of
-    the row sum, the logarithm's own rounding about 1e-7. Measured: 3.0e-7, and 5.9e-6 with the terms added to the running sum one by one."""
+    the row sum, the logarithm's own rounding about 1e-7. Measured: 3.0e-7, and 5.9e-6 with the terms added to the running sum one
+    by one."""
     assert _row_sum_noise() <= 5e-7
