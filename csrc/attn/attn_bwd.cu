@@ -18,8 +18,9 @@
 // run in opposite phases (2,830 clk). The price is 64-wide products with both operands in shared memory, which run at
 // 48 clk per step instead of 32 (6 KB at 128 B/clk): 2,480 clk of MMA time per item in the dK/dV kernel, whose TMEM is
 // full. The dQ kernel has room for Q and dO in TMEM and pays nothing (2,110 -> 1,740 clk per item, MMA time 1,536).
-// Kernel times, 32 heads over 8 KV heads, causal (before -> now): dK/dV 1,140 -> 816 us at 8,192 tokens, 16.2 -> 13.6 ms
-// at 32,768; dQ 709 -> 635 us and 11.0 -> 9.5 ms (the GPU runs at its power cap at 32,768, 1.5 GHz).
+// Kernel times, 32 heads over 8 KV heads, causal (before -> now): dK/dV 1,140 -> 797 us at 8,192 tokens, 16.2 -> 13.4 ms
+// at 32,768; dQ 709 -> 620 us and 11.0 -> 9.4 ms (the GPU runs at its power cap at 32,768, 1.5 GHz); with a 4,096-token
+// window over 65,536 tokens dK/dV 14.6 -> 8.2 ms, dQ 8.9 ms.
 // Exponentials are the special-function unit's: taking every second pair as a polynomial on the FMA pipe made no difference
 // (28.4 -> 29.1 ms for the whole backward at 32,768 tokens at the time), since instruction issue and the cycle of an item
 // bound these kernels.

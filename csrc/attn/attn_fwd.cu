@@ -10,8 +10,10 @@
 //                GPU into local staging with plain P2P loads while the tiles compute
 // TMEM (512 columns): S0 | S1 | O0 | O1; S_i is two halves of 64 keys, each with its bf16 P written over its first
 // half, so that the softmax of one half runs beside the products of the other.
-// Measured, 32 heads over 8 KV heads, causal, in a loop (before -> now): 79 -> 74 us at 16 heads x 4,096 tokens, 562 ->
-// 531 us at 8,192, 8.34 -> 7.82 ms at 32,768; 4,096-token window over 65,536 tokens 5.74 -> 4.68 ms. Before, eight warps
+// Measured, 32 heads over 8 KV heads, causal, in a loop (before -> now): 152 -> 135 us at 4,096 tokens, 519 -> 484 us at
+// 8,192, 8.34 -> 7.82 ms at 32,768; 4,096-token window over 65,536 tokens 5.74 -> 4.68 ms. A sequence of one 128-token
+// block, whose two halves follow one another with nothing beside them, takes longer: 1,024 of them 45 -> 51 us (7 waves;
+// of 256 tokens 24.7 -> 20.6 us for 256). Before, eight warps
 // served both tiles in turn, 128 keys at a time, every role walked the mask, each tile paid an integer division per
 // warp, and a quarter of the exponentials were polynomials (7.82 -> 8.18 ms when put back: instruction issue and fixed
 // latencies bound the softmax warps now, the special-function unit is busy 57 % of the time, the tensor pipe 70 %).
